@@ -16,7 +16,7 @@
 #include <cfloat>
 #include <cstdint>
 
-#include "common.cuh"
+#include "gpt_oss_attn.cuh"
 
 namespace gb200 {
 
@@ -62,16 +62,18 @@ struct OssRope {
     float theta, factor, initial_context, beta_fast, beta_slow;
 };
 
-// One thread per (token, rotated head, frequency): the pair (d, d + half) shares its angle.
-__global__ void oss_rope_kernel(const float* __restrict__ x, const long long* __restrict__ positions, float* __restrict__ y, int tokens,
-                                OssRope o)
+// A thread owns one (token, frequency) and walks over heads: the angle's powf, logf, cosf and sinf - some hundreds of
+// instructions - are paid once for all of them instead of once per pair.  blockDim.y threads (and gridDim.y CTAs, when there
+// are few tokens) share the heads of a token.
+__global__ void __launch_bounds__(256) oss_rope_kernel(const float* __restrict__ x, const long long* __restrict__ positions,
+                                                       float* __restrict__ y, int tokens, OssRope o)
 {
     const int half = o.head_dim / 2, rot_heads = o.q_heads + o.kv_heads;
     const int packed = (o.q_heads + 2 * o.kv_heads) * o.head_dim;
-    const size_t idx = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    const size_t pairs = size_t(tokens) * rot_heads * half;
-    if (idx < pairs) {
-        const int frequency = int(idx % half), head = int((idx / half) % rot_heads), token = int(idx / (size_t(half) * rot_heads));
+    const int token = blockIdx.x, part = blockIdx.y * blockDim.y + threadIdx.y, parts = gridDim.y * blockDim.y;
+    const float* xr = x + size_t(token) * packed;
+    float* yr = y + size_t(token) * packed;
+    for (int frequency = threadIdx.x; frequency < half; frequency += blockDim.x) {
         const float pi = 3.14159265358979323846f;
         float inv = powf(o.theta, -2.f * frequency / o.head_dim), concentration = 1;
         if (o.factor > 1) {
@@ -83,90 +85,53 @@ __global__ void oss_rope_kernel(const float* __restrict__ x, const long long* __
         }
         const float angle = float(positions[token]) * inv;
         const float cosine = bfr(cosf(angle) * concentration), sine = bfr(sinf(angle) * concentration);
-        const size_t at = size_t(token) * packed + size_t(head) * o.head_dim + frequency;
-        const float a = x[at], b = x[at + half];
-        y[at] = bfr(bfr(a * cosine) + bfr(-b * sine));
-        y[at + half] = bfr(bfr(b * cosine) + bfr(a * sine));
+#pragma unroll 4
+        for (int head = part; head < rot_heads; head += parts) {
+            const int at = head * o.head_dim + frequency;
+            const float a = xr[at], b = xr[at + half];
+            yr[at] = bfr(bfr(a * cosine) + bfr(-b * sine));
+            yr[at + half] = bfr(bfr(b * cosine) + bfr(a * sine));
+        }
     }
     // the v part passes through
-    const size_t vcount = size_t(tokens) * o.kv_heads * o.head_dim;
-    for (size_t i = idx; i < vcount; i += size_t(gridDim.x) * blockDim.x) {
-        const size_t token = i / (size_t(o.kv_heads) * o.head_dim), c = i % (size_t(o.kv_heads) * o.head_dim);
-        const size_t at = token * packed + size_t(rot_heads) * o.head_dim + c;
-        y[at] = x[at];
-    }
+    const int v0 = rot_heads * o.head_dim;
+    for (int c = v0 + part * blockDim.x + threadIdx.x; c < packed; c += parts * blockDim.x) yr[c] = xr[c];
 }
 
-struct OssAttn {
-    const float* qkv;             // [batch * tokens, (q + 2 kv) * d], already rotated
-    __nv_bfloat16* keys;          // [layers][physical pages][page size][kv heads][d]
-    __nv_bfloat16* values;
-    const int* table;             // [batch, logical pages]
-    const int* lengths;           // [batch]: positions visible at decode
-    const int* starts;            // [batch]: position of the first new token
-    const int* active;            // [batch]
-    const float* sinks;           // [q heads]
-    float* out;                   // [batch * tokens, q * d]
-    float* part;                  // [batch, q heads, splits, 2 + d]
-    unsigned* counters;           // [batch, kv heads]
-    int batch, tokens, logical_pages, physical_pages;
-    int q_heads, kv_heads, head_dim, layer, page_size, window, prefill, splits;
-};
-
-__device__ __forceinline__ size_t oss_cache_offset(const OssAttn& p, int b, int position, int head)
-{
-    if (position < 0 || position / p.page_size >= p.logical_pages) return SIZE_MAX;
-    const int page = p.table[b * p.logical_pages + position / p.page_size];
-    if (page < 0 || page >= p.physical_pages) return SIZE_MAX;
-    return (((size_t(p.layer) * p.physical_pages + page) * p.page_size + position % p.page_size) * p.kv_heads + head) * p.head_dim;
-}
-
+// Appends the rows' k and v at positions starts[b] + t.  A thread takes kVec neighbouring values of k or v (8 when the head
+// size and the pointers allow it): one page lookup and one 16-byte store for eight of them.
+template <int kVec>
 __global__ void oss_write_kv_kernel(const OssAttn p)
 {
-    const int kv_width = p.kv_heads * p.head_dim, packed = (p.q_heads + 2 * p.kv_heads) * p.head_dim;
+    const int kv_width = p.kv_heads * p.head_dim, packed = (p.q_heads + 2 * p.kv_heads) * p.head_dim, pieces = 2 * kv_width / kVec;
     const size_t idx = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (idx >= size_t(p.batch) * p.tokens * kv_width) return;
-    const int row = int(idx / kv_width), b = row / p.tokens, t = row % p.tokens, d = int(idx % kv_width);
+    if (idx >= size_t(p.batch) * p.tokens * pieces) return;
+    const int row = int(idx / pieces), b = row / p.tokens, t = row % p.tokens, c = int(idx % pieces) * kVec, is_v = c >= kv_width;
+    const int d = is_v ? c - kv_width : c;
     if (!p.active[b]) return;
     const size_t off = oss_cache_offset(p, b, p.starts[b] + t, d / p.head_dim);
     if (off == SIZE_MAX) return;
-    p.keys[off + d % p.head_dim] = __float2bfloat16(p.qkv[size_t(row) * packed + p.q_heads * p.head_dim + d]);
-    p.values[off + d % p.head_dim] = __float2bfloat16(p.qkv[size_t(row) * packed + (p.q_heads + p.kv_heads) * p.head_dim + d]);
+    const float* src = p.qkv + size_t(row) * packed + p.q_heads * p.head_dim + c;
+    __nv_bfloat16* dst = (is_v ? p.values : p.keys) + off + d % p.head_dim;
+    if constexpr (kVec == 8) {
+        const float4 lo = __ldg(reinterpret_cast<const float4*>(src)), hi = __ldg(reinterpret_cast<const float4*>(src) + 1);
+        const __nv_bfloat162 v[4] = {__floats2bfloat162_rn(lo.x, lo.y), __floats2bfloat162_rn(lo.z, lo.w),
+                                     __floats2bfloat162_rn(hi.x, hi.y), __floats2bfloat162_rn(hi.z, hi.w)};
+        *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(v);
+    } else {
+        *dst = __float2bfloat16(*src);
+    }
 }
 
 // Any shape: one warp per (row, q head), online softmax in position order (the reference's baseline).
 __global__ void oss_attention_generic_kernel(const OssAttn p)
 {
-    const int lane = threadIdx.x & 31;
     const int task = int((size_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32);
     if (task >= p.batch * p.tokens * p.q_heads) return;
-    const int head = task % p.q_heads, row = task / p.q_heads, b = row / p.tokens, t = row % p.tokens;
-    const int packed = (p.q_heads + 2 * p.kv_heads) * p.head_dim;
-    float accum[8] = {};
-    const int end = p.prefill ? p.starts[b] + t + 1 : p.lengths[b];
-    const int begin = p.window ? max(0, end - p.window) : 0;
-    float maximum = p.sinks[head], sum = 1;
-    const float* q = p.qkv + size_t(row) * packed + head * p.head_dim;
-    if (p.active[b] && end > 0 && end <= p.logical_pages * p.page_size) {
-        for (int pos = begin; pos < end; ++pos) {
-            const size_t off = oss_cache_offset(p, b, pos, head / (p.q_heads / p.kv_heads));
-            if (off == SIZE_MAX) continue;
-            float score = 0;
-            for (int d = lane; d < p.head_dim; d += 32) score += q[d] * __bfloat162float(p.keys[off + d]);
-            score = warp_sum(score) * rsqrtf(float(p.head_dim));
-            const float next = fmaxf(maximum, score);
-            const float old = expf(maximum - next), weight = expf(score - next);
-            sum = sum * old + weight;
-            for (int d = lane, i = 0; d < p.head_dim; d += 32, ++i) accum[i] = accum[i] * old + weight * __bfloat162float(p.values[off + d]);
-            maximum = next;
-        }
-    }
-    for (int d = lane, i = 0; d < p.head_dim; d += 32, ++i)
-        p.out[size_t(row) * p.q_heads * p.head_dim + head * p.head_dim + d] = bfr(accum[i] / sum);
+    oss_attention_row(p, task / p.q_heads, task % p.q_heads, threadIdx.x & 31);
 }
 
 constexpr int kOssSplit = 64;      // positions per split
-constexpr int kOssDim = 64;        // head dimension of the grouped decode kernel
 constexpr int kOssRowStride = 68;  // halves per staged row: 136 bytes (8-byte aligned), two-way bank conflicts at most
 
 // Decode (one new token per sequence), head_dim 64: CTA (kv head, split, sequence); warp g serves q head kv * group + g.
@@ -390,8 +355,11 @@ int garnet_b200_gpt_oss_rope(const garnet_b200_gpt_oss_options* o, const float* 
     if (int rc = validate_oss(o, false)) return rc;
     if (!d_x || !d_positions || !d_y || tokens <= 0) return fail(GARNET_B200_INVALID_VALUE, "gpt_oss_rope: bad argument");
     OssRope r{o->q_heads, o->kv_heads, o->head_dim, o->theta, o->factor, o->initial_context, o->beta_fast, o->beta_slow};
-    const size_t pairs = size_t(tokens) * (o->q_heads + o->kv_heads) * (o->head_dim / 2);
-    oss_rope_kernel<<<unsigned((pairs + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(d_x, d_positions, d_y, tokens, r);
+    const dim3 block(32, 8);
+    // about two CTAs per SM at least: a decode batch shares the heads of a token over several CTAs
+    const int heads = o->q_heads + o->kv_heads;
+    const unsigned parts = unsigned(std::max(1, std::min((heads + 7) / 8, 2 * kSmCount / tokens)));
+    oss_rope_kernel<<<dim3(unsigned(tokens), parts), block, 0, static_cast<cudaStream_t>(stream)>>>(d_x, d_positions, d_y, tokens, r);
     GB_CUDA(cudaGetLastError());
     return GARNET_B200_OK;
 }
@@ -428,8 +396,11 @@ int garnet_b200_gpt_oss_attention(const garnet_b200_gpt_oss_options* o, const vo
     p.splits = oss_splits(*o, logical_pages);
     p.part = nullptr, p.counters = nullptr;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const size_t n = size_t(batch) * tokens * o->kv_heads * o->head_dim;
-    oss_write_kv_kernel<<<unsigned((n + 255) / 256), 256, 0, s>>>(p);
+    const bool wide = o->head_dim % 8 == 0 && ((reinterpret_cast<uintptr_t>(in[0]) | reinterpret_cast<uintptr_t>(in[1]) |
+                                                reinterpret_cast<uintptr_t>(in[2])) & 15) == 0;
+    const size_t n = size_t(batch) * tokens * 2 * o->kv_heads * o->head_dim / (wide ? 8 : 1);
+    if (wide) oss_write_kv_kernel<8><<<unsigned((n + 255) / 256), 256, 0, s>>>(p);
+    else oss_write_kv_kernel<1><<<unsigned((n + 255) / 256), 256, 0, s>>>(p);
     GB_CUDA(cudaGetLastError());
     const int group = o->q_heads / o->kv_heads;
     const bool grouped = tokens == 1 && !o->prefill && o->head_dim == kOssDim && group <= 16 && in[4] &&
@@ -444,6 +415,7 @@ int garnet_b200_gpt_oss_attention(const garnet_b200_gpt_oss_options* o, const vo
     } else {
         if (!in[4] && !o->prefill) return fail(GARNET_B200_INVALID_VALUE, "gpt_oss_attention: decode needs the lengths operand");
         if (o->head_dim > 256) return fail(GARNET_B200_NOT_SUPPORTED, "gpt_oss_attention: head_dim above 256");
+        if (oss_prefill_takes(p)) return oss_prefill_launch(p, s);
         const size_t tasks = size_t(batch) * tokens * o->q_heads;
         oss_attention_generic_kernel<<<unsigned((tasks * 32 + 255) / 256), 256, 0, s>>>(p);
     }
