@@ -14,10 +14,8 @@ struct OssAttn {
     const int* active;            // [batch]
     const float* sinks;           // [q heads]
     float* out;                   // [batch * tokens, q * d]
-    float* part;                  // [batch, q heads, splits, 2 + d]
-    unsigned* counters;           // [batch, kv heads]
     int batch, tokens, logical_pages, physical_pages;
-    int q_heads, kv_heads, head_dim, layer, page_size, window, prefill, splits;
+    int q_heads, kv_heads, head_dim, layer, page_size, window, prefill;
 };
 
 #if defined(__CUDACC__)
@@ -58,6 +56,17 @@ __device__ __forceinline__ void oss_attention_row(const OssAttn& p, int row, int
     for (int d = lane, i = 0; d < p.head_dim; d += 32, ++i)
         p.out[size_t(row) * p.q_heads * p.head_dim + head * p.head_dim + d] = bf16_round_f(accum[i] / sum);
 }
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ uint32_t bf16x2_of(float lo, float hi)
+{
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
 #endif
 
 // gpt_oss_prefill.cu: many query rows of 64-wide heads on the tensor cores.  `oss_prefill_takes` says whether the shape and
@@ -65,5 +74,8 @@ __device__ __forceinline__ void oss_attention_row(const OssAttn& p, int row, int
 constexpr int kOssDim = 64;
 bool oss_prefill_takes(const OssAttn& p);
 int oss_prefill_launch(const OssAttn& p, cudaStream_t stream);
+// gpt_oss_decode.cu: one new token per sequence, 64-wide heads, up to 16 q heads per kv head.
+bool oss_decode_takes(const OssAttn& p);
+int oss_decode_launch(const OssAttn& p, cudaStream_t stream);
 
 }  // namespace gb200

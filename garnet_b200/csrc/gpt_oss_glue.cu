@@ -8,11 +8,8 @@
 // softmax denominator only), decodeAttentionPartial / Merge :376-428,:513-535, vocabTop1 :430-455,
 // the entry points RunGptOssRmsNorm / Rope / Attention / VocabTop1 :930-1210; decodeGemv
 // (plugins/gpt_oss/cuda/gpt_oss_gemv.cu:7-39).
-//
-// Decode attention here: one CTA per (kv head, 64-position split, sequence) stages the split's K
-// and V rows in shared memory once and serves all the q heads of the group from them (the
-// reference's default path reads them once per q head); the last CTA of a (sequence, kv head)
-// merges the splits and the sink.  With a sliding window of 128 a layer needs two splits.
+// Attention itself: gpt_oss_decode.cu (one token per sequence), gpt_oss_prefill.cu (many rows) and, for other shapes, the
+// row loop here.
 #include <cfloat>
 #include <cstdint>
 
@@ -29,13 +26,6 @@ __device__ __forceinline__ float warp_sum(float v)
     for (int off = 16; off; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
     return v;
 }
-__device__ __forceinline__ float warp_max(float v)
-{
-#pragma unroll
-    for (int off = 16; off; off >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, off));
-    return v;
-}
-
 // y = bf((bf(x) * rsqrt(mean(bf(x)^2) + eps)) * w), one CTA per row.
 __global__ void __launch_bounds__(256) oss_rms_norm_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y,
                                                            int hidden, float eps)
@@ -62,18 +52,25 @@ struct OssRope {
     float theta, factor, initial_context, beta_fast, beta_slow;
 };
 
-// A thread owns one (token, frequency) and walks over heads: the angle's powf, logf, cosf and sinf - some hundreds of
-// instructions - are paid once for all of them instead of once per pair.  blockDim.y threads (and gridDim.y CTAs, when there
-// are few tokens) share the heads of a token.
-__global__ void __launch_bounds__(256) oss_rope_kernel(const float* __restrict__ x, const long long* __restrict__ positions,
-                                                       float* __restrict__ y, int tokens, OssRope o)
+// A CTA rotates two tokens (or a share of one token's heads, when there are few): one thread per (token, frequency)
+// computes the angle's powf, logf, cosf and sinf - some hundreds of instructions - once for all heads, then every thread moves
+// kVec neighbouring frequencies of a head (16-byte loads and stores when the head size and the pointers allow it).
+// Bound: HBM, 2 x 4 bytes per value.  2048 tokens of 64 / 8 heads of 64 (84 MB): 24.0 -> 19.3 us (ncu) against one
+// thread per (token, frequency) and eight walking over the heads with 4-byte accesses.
+constexpr int kRopeTokens = 2, kRopeThreads = 256, kRopeMaxHalf = 128;
+
+template <int kVec, int kUnroll>
+__global__ void __launch_bounds__(kRopeThreads) oss_rope_kernel(const float* __restrict__ x, const long long* __restrict__ positions,
+                                                                float* __restrict__ y, int tokens, int per_cta, OssRope o)
 {
+    __shared__ __align__(16) float cosines[kRopeTokens][kRopeMaxHalf], sines[kRopeTokens][kRopeMaxHalf];
     const int half = o.head_dim / 2, rot_heads = o.q_heads + o.kv_heads;
     const int packed = (o.q_heads + 2 * o.kv_heads) * o.head_dim;
-    const int token = blockIdx.x, part = blockIdx.y * blockDim.y + threadIdx.y, parts = gridDim.y * blockDim.y;
-    const float* xr = x + size_t(token) * packed;
-    float* yr = y + size_t(token) * packed;
-    for (int frequency = threadIdx.x; frequency < half; frequency += blockDim.x) {
+    const int token0 = blockIdx.x * per_cta, count = min(per_cta, tokens - token0);
+    pdl_launch_dependents();
+    pdl_wait();
+    for (int i = threadIdx.x; i < count * half; i += kRopeThreads) {
+        const int token = i / half, frequency = i % half;
         const float pi = 3.14159265358979323846f;
         float inv = powf(o.theta, -2.f * frequency / o.head_dim), concentration = 1;
         if (o.factor > 1) {
@@ -83,19 +80,45 @@ __global__ void __launch_bounds__(256) oss_rope_kernel(const float* __restrict__
             inv *= (1 - ramp) + ramp / o.factor;
             concentration = 1 + .1f * logf(o.factor);
         }
-        const float angle = float(positions[token]) * inv;
-        const float cosine = bfr(cosf(angle) * concentration), sine = bfr(sinf(angle) * concentration);
-#pragma unroll 4
-        for (int head = part; head < rot_heads; head += parts) {
-            const int at = head * o.head_dim + frequency;
-            const float a = xr[at], b = xr[at + half];
-            yr[at] = bfr(bfr(a * cosine) + bfr(-b * sine));
-            yr[at + half] = bfr(bfr(b * cosine) + bfr(a * sine));
+        const float angle = float(positions[token0 + token]) * inv;
+        cosines[token][frequency] = bfr(cosf(angle) * concentration);
+        sines[token][frequency] = bfr(sinf(angle) * concentration);
+    }
+    __syncthreads();
+    const int pieces = half / kVec, part = blockIdx.y * kRopeThreads + threadIdx.x, parts = gridDim.y * kRopeThreads;
+    const int v0 = rot_heads * o.head_dim;
+    for (int token = 0; token < count; ++token) {
+        const float* xr = x + size_t(token0 + token) * packed;
+        float* yr = y + size_t(token0 + token) * packed;
+#pragma unroll kUnroll
+        for (int i = part; i < rot_heads * pieces; i += parts) {
+            const int f = i % pieces * kVec, at = i / pieces * o.head_dim + f;
+            float a[kVec], b[kVec], ra[kVec], rb[kVec];
+            if constexpr (kVec == 4) {
+                *reinterpret_cast<float4*>(a) = __ldg(reinterpret_cast<const float4*>(xr + at));
+                *reinterpret_cast<float4*>(b) = __ldg(reinterpret_cast<const float4*>(xr + at + half));
+            } else {
+                a[0] = xr[at], b[0] = xr[at + half];
+            }
+#pragma unroll
+            for (int j = 0; j < kVec; ++j) {
+                const float cosine = cosines[token][f + j], sine = sines[token][f + j];
+                ra[j] = bfr(bfr(a[j] * cosine) + bfr(-b[j] * sine));
+                rb[j] = bfr(bfr(b[j] * cosine) + bfr(a[j] * sine));
+            }
+            if constexpr (kVec == 4) {
+                *reinterpret_cast<float4*>(yr + at) = *reinterpret_cast<const float4*>(ra);
+                *reinterpret_cast<float4*>(yr + at + half) = *reinterpret_cast<const float4*>(rb);
+            } else {
+                yr[at] = ra[0], yr[at + half] = rb[0];
+            }
+        }
+        // the v part passes through
+        for (int c = v0 + part * kVec; c < packed; c += parts * kVec) {
+            if constexpr (kVec == 4) *reinterpret_cast<float4*>(yr + c) = __ldg(reinterpret_cast<const float4*>(xr + c));
+            else yr[c] = xr[c];
         }
     }
-    // the v part passes through
-    const int v0 = rot_heads * o.head_dim;
-    for (int c = v0 + part * blockDim.x + threadIdx.x; c < packed; c += parts * blockDim.x) yr[c] = xr[c];
 }
 
 // Appends the rows' k and v at positions starts[b] + t.  A thread takes kVec neighbouring values of k or v (8 when the head
@@ -105,6 +128,8 @@ __global__ void oss_write_kv_kernel(const OssAttn p)
 {
     const int kv_width = p.kv_heads * p.head_dim, packed = (p.q_heads + 2 * p.kv_heads) * p.head_dim, pieces = 2 * kv_width / kVec;
     const size_t idx = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    pdl_launch_dependents();
+    pdl_wait();
     if (idx >= size_t(p.batch) * p.tokens * pieces) return;
     const int row = int(idx / pieces), b = row / p.tokens, t = row % p.tokens, c = int(idx % pieces) * kVec, is_v = c >= kv_width;
     const int d = is_v ? c - kv_width : c;
@@ -129,124 +154,6 @@ __global__ void oss_attention_generic_kernel(const OssAttn p)
     const int task = int((size_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32);
     if (task >= p.batch * p.tokens * p.q_heads) return;
     oss_attention_row(p, task / p.q_heads, task % p.q_heads, threadIdx.x & 31);
-}
-
-constexpr int kOssSplit = 64;      // positions per split
-constexpr int kOssRowStride = 68;  // halves per staged row: 136 bytes (8-byte aligned), two-way bank conflicts at most
-
-// Decode (one new token per sequence), head_dim 64: CTA (kv head, split, sequence); warp g serves q head kv * group + g.
-__global__ void __launch_bounds__(512) oss_attention_decode_kernel(const OssAttn p)
-{
-    __shared__ __align__(16) __nv_bfloat16 ks[kOssSplit * kOssRowStride], vs[kOssSplit * kOssRowStride];
-    __shared__ float qs[16][kOssDim];
-    __shared__ unsigned char row_ok[kOssSplit];   // the row's page exists (looked up once, while staging)
-    __shared__ int s_last;
-    const int kv = blockIdx.x, split = blockIdx.y, b = blockIdx.z;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, group = p.q_heads / p.kv_heads;
-    const int head = kv * group + warp;
-    const int packed = (p.q_heads + 2 * p.kv_heads) * kOssDim;
-    const int end = p.lengths[b];
-    const bool live = p.active[b] && end > 0 && end <= p.logical_pages * p.page_size;
-    const int begin = p.window ? max(0, end - p.window) : 0;
-    const int s0 = begin + split * kOssSplit, s1 = live ? min(end, s0 + kOssSplit) : s0;
-    const int rows = max(0, s1 - s0);
-    // ---- stage the split's K and V rows: 8 pieces of 16 bytes per row and tensor
-    for (int i = threadIdx.x; i < rows * 16; i += blockDim.x) {
-        const int r = i >> 4, piece = i & 7, is_v = (i >> 3) & 1;
-        const size_t off = oss_cache_offset(p, b, s0 + r, kv);
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (off != SIZE_MAX) v = __ldcg(reinterpret_cast<const uint4*>((is_v ? p.values : p.keys) + off) + piece);
-        if ((i & 15) == 0) row_ok[r] = off != SIZE_MAX;
-        // a staged row starts on an 8-byte boundary (136-byte rows): two 8-byte stores
-        uint2* dst = reinterpret_cast<uint2*>((is_v ? vs : ks) + r * kOssRowStride + piece * 8);
-        dst[0] = make_uint2(v.x, v.y);
-        dst[1] = make_uint2(v.z, v.w);
-    }
-    {
-        const float* qg = p.qkv + size_t(b) * packed + head * kOssDim;
-        qs[warp][lane] = qg[lane];
-        qs[warp][lane + 32] = qg[lane + 32];
-    }
-    __syncthreads();
-    const float* q = qs[warp];
-    const float scale = rsqrtf(float(kOssDim));
-    // ---- scores: lane owns rows lane and lane + 32
-    float sc[2];
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-        const int r = lane + 32 * u;
-        float s = -FLT_MAX;
-        if (r < rows && row_ok[r]) {
-            float acc = 0.f;
-            const __nv_bfloat162* kr = reinterpret_cast<const __nv_bfloat162*>(ks + r * kOssRowStride);
-#pragma unroll 8
-            for (int d = 0; d < kOssDim / 2; ++d) {
-                const float2 kk = __bfloat1622float2(kr[d]);
-                acc += q[2 * d] * kk.x + q[2 * d + 1] * kk.y;
-            }
-            s = acc * scale;
-        }
-        sc[u] = s;
-    }
-    const float m = warp_max(fmaxf(sc[0], sc[1]));
-    float w[2], out0 = 0.f, out1 = 0.f;
-#pragma unroll
-    for (int u = 0; u < 2; ++u) w[u] = sc[u] > -FLT_MAX ? __expf(sc[u] - m) : 0.f;
-    const float total = warp_sum(w[0] + w[1]);
-    // ---- weighted values: lane owns dims 2 lane, 2 lane + 1
-    for (int r = 0; r < rows; ++r) {
-        const float wr = __shfl_sync(0xffffffffu, w[r >> 5], r & 31);
-        const float2 vv = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(vs + r * kOssRowStride)[lane]);
-        out0 += wr * vv.x;
-        out1 += wr * vv.y;
-    }
-    const size_t pi = ((size_t(b) * p.q_heads + head) * p.splits + split) * (2 + kOssDim);
-    if (warp < group) {
-        if (lane == 0) p.part[pi] = total > 0.f ? m : -FLT_MAX, p.part[pi + 1] = total;
-        p.part[pi + 2 + 2 * lane] = out0;
-        p.part[pi + 3 + 2 * lane] = out1;
-    }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(&p.counters[b * p.kv_heads + kv], 1u) == unsigned(p.splits) - 1u;
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    // ---- merge the splits of this group's heads, and the sink (denominator only)
-    if (warp < group) {
-        const size_t hb = (size_t(b) * p.q_heads + head) * p.splits * (2 + kOssDim);
-        float mx = p.sinks[head];
-        for (int s = lane; s < p.splits; s += 32) {   // both values requested at once
-            const float pmax = __ldcg(&p.part[hb + size_t(s) * (2 + kOssDim)]), psum = __ldcg(&p.part[hb + size_t(s) * (2 + kOssDim) + 1]);
-            if (psum > 0.f) mx = fmaxf(mx, pmax);
-        }
-        mx = warp_max(mx);
-        float sum = __expf(p.sinks[head] - mx), o0 = 0.f, o1 = 0.f;
-        // eight splits' values are requested together, without a condition on them, so that the loads overlap
-        // instead of queueing behind one another (the order of the additions stays the order of the splits)
-        for (int sb = 0; sb < p.splits; sb += 8) {
-            float pm[8], psum[8], po0[8], po1[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const bool in = sb + u < p.splits;
-                const float* ps = p.part + hb + size_t(in ? sb + u : sb) * (2 + kOssDim);
-                pm[u] = __ldcg(ps), psum[u] = in ? __ldcg(ps + 1) : 0.f;
-                po0[u] = __ldcg(ps + 2 + 2 * lane), po1[u] = __ldcg(ps + 3 + 2 * lane);
-            }
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                if (psum[u] <= 0.f) continue;
-                const float f = __expf(pm[u] - mx);
-                sum += f * psum[u];
-                o0 += f * po0[u];
-                o1 += f * po1[u];
-            }
-        }
-        float* o = p.out + size_t(b) * p.q_heads * kOssDim + head * kOssDim;
-        o[2 * lane] = bfr(live ? o0 / sum : 0.f);
-        o[2 * lane + 1] = bfr(live ? o1 / sum : 0.f);
-    }
-    if (threadIdx.x == 0) p.counters[b * p.kv_heads + kv] = 0;
 }
 
 __global__ void __launch_bounds__(256) oss_vocab_top1_kernel(const float* __restrict__ logits, float* __restrict__ pairs, int width, int rank)
@@ -320,16 +227,30 @@ int validate_oss(const garnet_b200_gpt_oss_options* o, bool attention)
     return GARNET_B200_OK;
 }
 
-int oss_splits(const garnet_b200_gpt_oss_options& o, int logical_pages)
-{
-    const int span = o.window ? std::min(o.window, logical_pages * o.page_size) : logical_pages * o.page_size;
-    return std::max(1, (span + kOssSplit - 1) / kOssSplit);
-}
-
+// The workspace that a decode call brings: a counter per (sequence, kv head) and a record of 2 + 64 numbers per (q head, 64
+// positions).  The size is part of the interface; the decode kernel merges its splits on the chip and leaves it alone.
 size_t oss_workspace(const garnet_b200_gpt_oss_options& o, int batch, int logical_pages)
 {
+    const int span = o.window ? std::min(o.window, logical_pages * o.page_size) : logical_pages * o.page_size;
+    const int splits = std::max(1, (span + 63) / 64);
     const size_t counters = (size_t(batch) * o.kv_heads * 4 + 255) & ~size_t(255);
-    return counters + size_t(batch) * o.q_heads * oss_splits(o, logical_pages) * (2 + kOssDim) * 4;
+    return counters + size_t(batch) * o.q_heads * splits * (2 + kOssDim) * 4;
+}
+
+// A launch that may start while the kernel before it drains (its griddepcontrol.wait is where it waits for that kernel).
+template <typename... Params, typename... Args>
+cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, int threads, cudaStream_t stream, Args... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(unsigned(threads));
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
 }
 
 }  // namespace
@@ -355,12 +276,15 @@ int garnet_b200_gpt_oss_rope(const garnet_b200_gpt_oss_options* o, const float* 
     if (int rc = validate_oss(o, false)) return rc;
     if (!d_x || !d_positions || !d_y || tokens <= 0) return fail(GARNET_B200_INVALID_VALUE, "gpt_oss_rope: bad argument");
     OssRope r{o->q_heads, o->kv_heads, o->head_dim, o->theta, o->factor, o->initial_context, o->beta_fast, o->beta_slow};
-    const dim3 block(32, 8);
     // about two CTAs per SM at least: a decode batch shares the heads of a token over several CTAs
-    const int heads = o->q_heads + o->kv_heads;
-    const unsigned parts = unsigned(std::max(1, std::min((heads + 7) / 8, 2 * kSmCount / tokens)));
-    oss_rope_kernel<<<dim3(unsigned(tokens), parts), block, 0, static_cast<cudaStream_t>(stream)>>>(d_x, d_positions, d_y, tokens, r);
-    GB_CUDA(cudaGetLastError());
+    const bool wide = o->head_dim % 8 == 0 && ((reinterpret_cast<uintptr_t>(d_x) | reinterpret_cast<uintptr_t>(d_y)) & 15) == 0;
+    const int items = (o->q_heads + o->kv_heads) * o->head_dim / (wide ? 8 : 2), per_cta = tokens < 2 * kSmCount ? 1 : kRopeTokens,
+              blocks = (tokens + per_cta - 1) / per_cta;
+    const unsigned parts = unsigned(std::max(1, std::min((items + kRopeThreads - 1) / kRopeThreads, 2 * kSmCount / blocks)));
+    // few tokens: little code, since a thread has one piece and fetches its instructions cold (4 tokens 7.4 -> 6.1 us)
+    const auto kernel = !wide ? oss_rope_kernel<1, 1> : per_cta == 1 ? oss_rope_kernel<4, 1> : oss_rope_kernel<4, 3>;
+    GB_CUDA(launch_dependent(kernel, dim3(unsigned(blocks), parts), kRopeThreads,
+                             static_cast<cudaStream_t>(stream), d_x, d_positions, d_y, tokens, per_cta, r));
     return GARNET_B200_OK;
 }
 
@@ -393,32 +317,25 @@ int garnet_b200_gpt_oss_attention(const garnet_b200_gpt_oss_options* o, const vo
     p.batch = batch, p.tokens = tokens, p.logical_pages = logical_pages, p.physical_pages = physical_pages;
     p.q_heads = o->q_heads, p.kv_heads = o->kv_heads, p.head_dim = o->head_dim, p.layer = o->layer, p.page_size = o->page_size;
     p.window = o->window, p.prefill = o->prefill;
-    p.splits = oss_splits(*o, logical_pages);
-    p.part = nullptr, p.counters = nullptr;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const bool wide = o->head_dim % 8 == 0 && ((reinterpret_cast<uintptr_t>(in[0]) | reinterpret_cast<uintptr_t>(in[1]) |
                                                 reinterpret_cast<uintptr_t>(in[2])) & 15) == 0;
     const size_t n = size_t(batch) * tokens * 2 * o->kv_heads * o->head_dim / (wide ? 8 : 1);
-    if (wide) oss_write_kv_kernel<8><<<unsigned((n + 255) / 256), 256, 0, s>>>(p);
-    else oss_write_kv_kernel<1><<<unsigned((n + 255) / 256), 256, 0, s>>>(p);
-    GB_CUDA(cudaGetLastError());
+    GB_CUDA(launch_dependent(wide ? oss_write_kv_kernel<8> : oss_write_kv_kernel<1>, dim3(unsigned((n + 255) / 256)), 256, s, p));
     const int group = o->q_heads / o->kv_heads;
     const bool grouped = tokens == 1 && !o->prefill && o->head_dim == kOssDim && group <= 16 && in[4] &&
                          (reinterpret_cast<uintptr_t>(in[1]) & 15) == 0 && (reinterpret_cast<uintptr_t>(in[2]) & 15) == 0;
     if (grouped) {
         if (!d_workspace || workspace_bytes < oss_workspace(*o, batch, logical_pages) || (reinterpret_cast<uintptr_t>(d_workspace) & 255))
             return fail(GARNET_B200_INVALID_VALUE, "gpt_oss_attention: the workspace is missing, too small or not 256-byte aligned");
-        uint8_t* ws = static_cast<uint8_t*>(d_workspace);
-        p.counters = reinterpret_cast<unsigned*>(ws);
-        p.part = reinterpret_cast<float*>(ws + ((size_t(batch) * o->kv_heads * 4 + 255) & ~size_t(255)));
-        oss_attention_decode_kernel<<<dim3(unsigned(o->kv_heads), unsigned(p.splits), unsigned(batch)), std::max(group, 1) * 32, 0, s>>>(p);
+        if (oss_decode_takes(p)) return oss_decode_launch(p, s);
     } else {
         if (!in[4] && !o->prefill) return fail(GARNET_B200_INVALID_VALUE, "gpt_oss_attention: decode needs the lengths operand");
         if (o->head_dim > 256) return fail(GARNET_B200_NOT_SUPPORTED, "gpt_oss_attention: head_dim above 256");
-        if (oss_prefill_takes(p)) return oss_prefill_launch(p, s);
-        const size_t tasks = size_t(batch) * tokens * o->q_heads;
-        oss_attention_generic_kernel<<<unsigned((tasks * 32 + 255) / 256), 256, 0, s>>>(p);
     }
+    if (oss_prefill_takes(p)) return oss_prefill_launch(p, s);
+    const size_t tasks = size_t(batch) * tokens * o->q_heads;
+    oss_attention_generic_kernel<<<unsigned((tasks * 32 + 255) / 256), 256, 0, s>>>(p);
     GB_CUDA(cudaGetLastError());
     return GARNET_B200_OK;
 }

@@ -46,21 +46,11 @@ struct PfSmem {
     static constexpr int total = bars + 128 + 1024;                // barriers, and slack for 1024-byte alignment
 };
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid)
-{
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
-}
 __device__ __forceinline__ float ex2(float x)
 {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
-}
-__device__ __forceinline__ uint32_t bf16x2_of(float lo, float hi)
-{
-    uint32_t r;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
-    return r;
 }
 // D[tmem] (+)= A[tmem] * B[smem]; issued by one thread.
 __device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, bool accumulate)

@@ -1,0 +1,75 @@
+"""gpt-oss decode attention (gpt_oss_decode.cu) against a float64 restatement of RunGptOssAttention
+(plugins/gpt_oss/cuda/gpt_oss_kernels.cu:125-160,376-535), at the sizes where its tiles of 16 positions, rounds of
+warps and clusters can go wrong, and RoPE's two access widths against each other."""
+import math
+
+import pytest
+import torch
+
+from garnet_b200 import gpt_oss as go
+from test_gpt_oss_prefill_gpu import D, check, make, run, want
+
+pytestmark = pytest.mark.gpu
+
+
+def decode(starts, window=0, **kw):
+    return make(1, starts, window, prefill=0, **kw)
+
+
+@pytest.mark.parametrize("starts,window", [
+    ([0], 0), ([14, 15, 16], 0), ([126, 127, 128], 0), ([254, 255, 256, 511, 512, 1023], 0), ([3071, 3072, 383], 0),
+    ([8190, 0], 0), ([0, 1, 500], 1), ([126, 127, 128, 2000], 128), ([300, 5], 129), (list(range(100, 500, 17)), 0),
+    (list(range(100, 500, 17)) * 6, 200)])
+def test_lengths_and_windows(starts, window):
+    check(decode(starts, window))
+
+
+@pytest.mark.parametrize("q_heads,kv_heads,page", [(8, 8, 16), (8, 4, 5), (6, 2, 16), (16, 1, 1), (48, 4, 32), (34, 2, 16)])
+def test_head_groups_and_page_sizes(q_heads, kv_heads, page):
+    check(decode([200, 7, 1500], 0, q_heads=q_heads, kv_heads=kv_heads, page=page))
+
+
+def test_sinks_large_scores_and_queries_that_are_not_bf16_values():
+    c = decode([700, 63], 0, scale=3.0, seed=2)
+    c["sinks"][::3] = 30.0
+    c["sinks"][1::3] = -math.inf
+    check(c)
+    check(decode([700, 63], 0, exact=False, seed=4))
+
+
+def test_inactive_sequences_missing_pages_and_positions_beyond_the_table():
+    c = decode([90, 10, 130, 0, 60], 0, seed=3)
+    c["active"][1] = 0
+    c["table"][0, 1] = -1
+    c["table"][0, 4] = c["physical"]
+    c["table"][4, :] = -1                              # nothing but the sink
+    c["table"] = c["table"][:, :7].contiguous()        # sequence 2 ends past the last logical page
+    check(c)
+
+
+def test_infinite_values_stay_infinite():
+    c = decode([300, 40], 0, seed=5)
+    slot = c["table"][0, 3]
+    c["values"][1, slot, 2, 0, 7] = math.inf
+    c["values"][1, slot, 5, 1, 9] = -math.inf
+    got, (w, _) = run(c).to(D).reshape(2, 64, 64), want(c)
+    w = w.reshape(2, 64, 64)
+    assert bool((got[0, :8, 7] == math.inf).all()) and bool((got[0, 8:16, 9] == -math.inf).all())
+    rest = torch.isfinite(w)
+    assert torch.equal(torch.isfinite(got), rest) and float((got - w)[rest].abs().max()) < 2e-2
+
+
+def test_operands_that_are_not_aligned_take_the_row_loop():
+    c = decode([100, 33], 0, seed=6)
+    buf = torch.empty(c["qkv"].numel() + 1, device="cuda")
+    moved = buf[1:].view_as(c["qkv"]).copy_(c["qkv"])
+    check(dict(c, qkv=moved))
+
+
+def test_rope_access_widths_agree():
+    opt = go.options(q_heads=6, kv_heads=2, head_dim=64)
+    for tokens in (1, 2, 3, 77, 301):
+        x = torch.randn(tokens, 10 * 64, device="cuda").to(torch.bfloat16).float()
+        positions = torch.randint(0, 9000, (tokens,), device="cuda")
+        moved = torch.empty(x.numel() + 1, device="cuda")[1:].view_as(x).copy_(x)
+        assert torch.equal(go.rope(opt, x, positions), go.rope(opt, moved, positions))
