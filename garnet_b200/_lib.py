@@ -7,6 +7,8 @@ from __future__ import annotations
 import ctypes
 import os
 
+import torch
+
 from . import _build
 
 OK, INVALID_VALUE, NOT_SUPPORTED, CUDA_ERROR, DEVICE_FAULT, OUT_OF_MEMORY = range(6)
@@ -140,3 +142,9 @@ def lib() -> ctypes.CDLL:
 def check(code: int) -> None:
     if code != OK:
         raise GarnetB200Error(code, lib().garnet_b200_last_error().decode())
+
+
+def stream_ptr() -> int:
+    """Handle of the current stream of the current device.  Asked for by its raw handle: building a
+    torch.cuda.Stream object for it took 3.2 us of a call whose kernel runs 6 us."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())

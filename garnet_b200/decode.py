@@ -27,7 +27,7 @@ from dataclasses import dataclass
 import numpy as np
 import torch
 
-from ._lib import check, lib
+from ._lib import check, lib, stream_ptr
 from .linear import GlueList, W4A16Linear
 
 
@@ -64,10 +64,6 @@ def rope_tables(positions: int, head_dim: int, theta: float):
     return np.cos(ang).astype(np.float32), np.sin(ang).astype(np.float32)
 
 
-def _stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
-
-
 class PagedAttention:
     """garnet_b200_attention_decode with its workspace."""
 
@@ -85,19 +81,19 @@ class PagedAttention:
         check(lib().garnet_b200_attention_decode(ctypes.byref(self.opt), qkv.data_ptr(), q_norm_w.data_ptr(), k_norm_w.data_ptr(),
                                                  cos.data_ptr(), sin.data_ptr(), key_pages.data_ptr(), value_pages.data_ptr(),
                                                  page_tables.data_ptr(), positions.data_ptr(), out.data_ptr(), self.ws.data_ptr(),
-                                                 self.ws.numel(), self.batch, 1 if pdl else 0, _stream_ptr()))
+                                                 self.ws.numel(), self.batch, 1 if pdl else 0, stream_ptr()))
         return out
 
 
 def embedding_gather(table, ids, out, pdl: bool = False):
     check(lib().garnet_b200_embedding_gather(table.data_ptr(), ids.data_ptr(), out.data_ptr(), ids.numel(), table.shape[1],
-                                             table.shape[0], 1 if pdl else 0, _stream_ptr()))
+                                             table.shape[0], 1 if pdl else 0, stream_ptr()))
     return out
 
 
 def argmax_bf16(logits, out, pdl: bool = False):
     check(lib().garnet_b200_argmax_bf16(logits.data_ptr(), out.data_ptr(), logits.shape[0], logits.shape[1], 1 if pdl else 0,
-                                        _stream_ptr()))
+                                        stream_ptr()))
     return out
 
 

@@ -23,13 +23,9 @@ import numpy as np
 import torch
 import torch.distributed as dist
 
-from ._lib import BF16, FP32, check, lib
+from ._lib import BF16, FP32, check, lib, stream_ptr
 
 BLOB_BYTES = 128
-
-
-def _stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
 
 
 class Comm:
@@ -57,7 +53,7 @@ class Comm:
         return lib().garnet_b200_comm_fault(self._c)
 
     def selftest_wait(self, limit_ms: int = 20) -> int:
-        return lib().garnet_b200_comm_selftest_wait(self._c, limit_ms, _stream_ptr())
+        return lib().garnet_b200_comm_selftest_wait(self._c, limit_ms, stream_ptr())
 
     def close(self) -> None:
         if self._c:
@@ -76,19 +72,19 @@ class Channel:
     def all_gather(self, src: torch.Tensor, dst: torch.Tensor) -> torch.Tensor:
         """dst[r] = src of rank r (dst: [world, *src.shape], contiguous)."""
         nbytes = src.numel() * src.element_size()
-        check(lib().garnet_b200_comm_all_gather(self._h, src.data_ptr(), nbytes, dst.data_ptr(), _stream_ptr()))
+        check(lib().garnet_b200_comm_all_gather(self._h, src.data_ptr(), nbytes, dst.data_ptr(), stream_ptr()))
         return dst
 
     def all_reduce(self, src: torch.Tensor, dst: torch.Tensor, wire: torch.dtype = torch.float32) -> torch.Tensor:
         """dst = sum over ranks of src (fp32 tensors); `wire` bf16 sends bf16 and rounds the sum to bf16."""
         check(lib().garnet_b200_comm_all_reduce(self._h, src.data_ptr(), dst.data_ptr(), src.numel(),
-                                                BF16 if wire == torch.bfloat16 else FP32, _stream_ptr()))
+                                                BF16 if wire == torch.bfloat16 else FP32, stream_ptr()))
         return dst
 
 
     def all_reduce_bf16(self, src: torch.Tensor, dst: torch.Tensor) -> torch.Tensor:
         """dst = bf16(sum over ranks of src), bf16 tensors; for two ranks exactly bf16(a + b)."""
-        check(lib().garnet_b200_comm_all_reduce_bf16(self._h, src.data_ptr(), dst.data_ptr(), src.numel(), _stream_ptr()))
+        check(lib().garnet_b200_comm_all_reduce_bf16(self._h, src.data_ptr(), dst.data_ptr(), src.numel(), stream_ptr()))
         return dst
 
 
@@ -110,7 +106,7 @@ class ExpertParallel:
     def run(self, x: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
         x2 = x.reshape(-1, self.moe.opt.hidden).contiguous()
         y = out if out is not None else torch.empty_like(x2)
-        check(lib().garnet_b200_moe_ep_run(self._e, x2.data_ptr(), y.data_ptr(), x2.shape[0], _stream_ptr()))
+        check(lib().garnet_b200_moe_ep_run(self._e, x2.data_ptr(), y.data_ptr(), x2.shape[0], stream_ptr()))
         return y
 
     def rows_received(self) -> int:

@@ -13,14 +13,15 @@ import ctypes
 import torch
 
 from . import _lib
-from ._lib import BF16, FP16, FP32, check, lib
+from ._lib import BF16, FP16, FP32, check, lib, stream_ptr
 
 _SCALE_KIND = {torch.float16: FP16, torch.bfloat16: BF16}
 _SRC_KIND = {torch.float16: FP16, torch.bfloat16: BF16, torch.float32: FP32}
 
 
-def _stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+def _rows(x: torch.Tensor, k: int) -> torch.Tensor:
+    """x as contiguous rows of k values; a tensor that is that already is taken as it is."""
+    return x if x.dim() == 2 and x.shape[1] == k and x.is_contiguous() else x.reshape(-1, k).contiguous()
 
 
 def quantize_int4(weight: torch.Tensor, group: int = 128, scale_dtype: torch.dtype = torch.bfloat16):
@@ -34,7 +35,7 @@ def quantize_int4(weight: torch.Tensor, group: int = 128, scale_dtype: torch.dty
     scales = torch.empty(rows, cols // group, dtype=scale_dtype, device=w.device)
     check(lib().garnet_b200_int4_quantize(w.data_ptr(), _SRC_KIND[w.dtype], rows, cols, group,
                                           _SCALE_KIND[scale_dtype], nibbles.data_ptr(), scales.data_ptr(),
-                                          _stream_ptr()))
+                                          stream_ptr()))
     return nibbles, scales
 
 
@@ -62,7 +63,7 @@ def forward_group(linears, x: torch.Tensor, outs=None, pdl: bool = True):
         outs = [torch.empty(m, lin.n, dtype=torch.bfloat16, device=x.device) for lin in linears]
     hs = (ctypes.c_void_p * len(linears))(*[lin._h for lin in linears])
     ys = (ctypes.c_void_p * len(linears))(*[o.data_ptr() for o in outs])
-    check(lib().garnet_b200_w4a16_run_group(hs, len(linears), x2.data_ptr(), ys, m, 1 if pdl else 0, _stream_ptr()))
+    check(lib().garnet_b200_w4a16_run_group(hs, len(linears), x2.data_ptr(), ys, m, 1 if pdl else 0, stream_ptr()))
     return outs
 
 
@@ -82,7 +83,7 @@ class LinearList:
         check(lib().garnet_b200_w4a16_list_create(hs, xs, ys, deps, n, m, ctypes.byref(self._l)))
 
     def run(self, pdl: bool = False) -> None:
-        check(lib().garnet_b200_w4a16_list_run(self._l, 1 if pdl else 0, _stream_ptr()))
+        check(lib().garnet_b200_w4a16_list_run(self._l, 1 if pdl else 0, stream_ptr()))
 
     def fault(self) -> int:
         return lib().garnet_b200_w4a16_list_fault(self._l)
@@ -145,7 +146,7 @@ class HostBatch:
         check(lib().garnet_b200_w4a16_batch_create(hs, xs, ys, ms, n, ctypes.byref(self._b)))
 
     def run(self) -> None:
-        check(lib().garnet_b200_w4a16_batch_run(self._b, _stream_ptr()))
+        check(lib().garnet_b200_w4a16_batch_run(self._b, stream_ptr()))
 
     def close(self) -> None:
         if self._b:
@@ -167,6 +168,7 @@ class W4A16Linear:
         self.n = self.k = self.group = 0
         self._keep = None
         self._ws = None
+        self._ws_need = (-1, 0)          # (rows, workspace bytes) of the last call
         self._host_rows = 0
 
     def reserve_host(self, max_m: int) -> None:
@@ -187,7 +189,7 @@ class W4A16Linear:
         h = ctypes.c_void_p(None)
         create = lib().garnet_b200_w4a16_create if shard_axis == 0 else lib().garnet_b200_w4a16_create_k_shard
         check(create(nb.data_ptr(), sc.data_ptr(), _SCALE_KIND[sc.dtype], n, k, group, shard_rank, shard_world,
-                     _stream_ptr(), ctypes.byref(h)))
+                     stream_ptr(), ctypes.byref(h)))
         self._h, self.group = h, group
         self.n = n // shard_world if shard_axis == 0 else n
         self.k = k // shard_world if shard_axis == 1 else k
@@ -209,7 +211,10 @@ class W4A16Linear:
         return out.value
 
     def _workspace(self, m: int, device) -> torch.Tensor | None:
-        need = self.workspace_bytes(m)
+        rows, need = self._ws_need
+        if rows != m:
+            need = self.workspace_bytes(m)
+            self._ws_need = (m, need)
         if need == 0:
             return None
         if self._ws is None or self._ws.numel() < need or self._ws.device != device:
@@ -221,20 +226,20 @@ class W4A16Linear:
                 pdl: bool = True) -> torch.Tensor:
         if x.dtype != torch.bfloat16 or not x.is_cuda:
             raise ValueError("forward needs a bf16 CUDA tensor")
-        x2 = x.reshape(-1, self.k).contiguous()
+        x2 = _rows(x, self.k)
         m = x2.shape[0]
         y = out if out is not None else torch.empty(m, self.n, dtype=torch.bfloat16, device=x.device)
         ws = workspace if workspace is not None else self._workspace(m, x.device)
         check(lib().garnet_b200_w4a16_run(self._h, x2.data_ptr(), y.data_ptr(), m,
                                           ws.data_ptr() if ws is not None else None,
-                                          ws.numel() if ws is not None else 0, 1 if pdl else 0, _stream_ptr()))
+                                          ws.numel() if ws is not None else 0, 1 if pdl else 0, stream_ptr()))
         return y
 
     def forward_host(self, x_host: torch.Tensor, y_host: torch.Tensor) -> torch.Tensor:
         """Host buffers in, host buffers out (copies inside the call)."""
         m = x_host.numel() // self.k
         self.reserve_host(m)
-        check(lib().garnet_b200_w4a16_run_host(self._h, x_host.data_ptr(), y_host.data_ptr(), m, _stream_ptr()))
+        check(lib().garnet_b200_w4a16_run_host(self._h, x_host.data_ptr(), y_host.data_ptr(), m, stream_ptr()))
         return y_host
 
     def forward_host_async(self, x_host: torch.Tensor, y_host: torch.Tensor) -> torch.Tensor:
@@ -242,12 +247,12 @@ class W4A16Linear:
         current stream has been synchronised."""
         m = x_host.numel() // self.k
         self.reserve_host(m)
-        check(lib().garnet_b200_w4a16_run_host_async(self._h, x_host.data_ptr(), y_host.data_ptr(), m, _stream_ptr()))
+        check(lib().garnet_b200_w4a16_run_host_async(self._h, x_host.data_ptr(), y_host.data_ptr(), m, stream_ptr()))
         return y_host
 
     def dequantized(self) -> torch.Tensor:
         out = torch.empty(self.n, self.k, dtype=torch.float32, device="cuda")
-        check(lib().garnet_b200_w4a16_dequant(self._h, out.data_ptr(), _stream_ptr()))
+        check(lib().garnet_b200_w4a16_dequant(self._h, out.data_ptr(), stream_ptr()))
         return out
 
     def fault(self) -> int:
@@ -259,6 +264,7 @@ class W4A16Linear:
             self._h = ctypes.c_void_p(None)
         self._keep = None
         self._ws = None
+        self._ws_need = (-1, 0)
         self._host_rows = 0
 
     def __del__(self):

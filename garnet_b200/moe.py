@@ -11,7 +11,7 @@ import ctypes
 
 import torch
 
-from ._lib import BF16, FP32, check, lib
+from ._lib import BF16, FP32, check, lib, stream_ptr
 
 
 class MoeOptions(ctypes.Structure):
@@ -24,10 +24,6 @@ class MoeOptions(ctypes.Structure):
 
 
 LAYOUT_BOTH, LAYOUT_STREAM, LAYOUT_BLOCK = 0, 1, 2
-
-
-def _stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
 
 
 class GptOssMoe:
@@ -64,7 +60,7 @@ class GptOssMoe:
             raise ValueError("prepare needs device-resident operands")
         arr = (ctypes.c_void_p * 8)(*[t.data_ptr() for t in tensors])
         h = ctypes.c_void_p(None)
-        check(lib().garnet_b200_moe_create(ctypes.byref(self.opt), arr, _stream_ptr(), ctypes.byref(h)))
+        check(lib().garnet_b200_moe_create(ctypes.byref(self.opt), arr, stream_ptr(), ctypes.byref(h)))
         self._h = h
         self._keep = tensors            # router weights and biases are borrowed by the handle
         return self
@@ -78,7 +74,7 @@ class GptOssMoe:
         arr = (ctypes.c_void_p * 4)(*[t.data_ptr() for t in small])
         blobs = (ctypes.c_void_p * 4)(*[(t.data_ptr() if t is not None else None) for t in packed])
         h = ctypes.c_void_p(None)
-        check(lib().garnet_b200_moe_create_prepacked(ctypes.byref(self.opt), arr, blobs, _stream_ptr(), ctypes.byref(h)))
+        check(lib().garnet_b200_moe_create_prepacked(ctypes.byref(self.opt), arr, blobs, stream_ptr(), ctypes.byref(h)))
         self._h = h
         self._keep = small + [t for t in packed if t is not None]
         return self
@@ -123,7 +119,7 @@ class GptOssMoe:
         y = out if out is not None else torch.empty_like(x2)
         ws = workspace if workspace is not None else self._workspace(tokens, x.device)
         check(lib().garnet_b200_moe_run(self._h, x2.data_ptr(), y.data_ptr(), ws.data_ptr(), ws.numel(), tokens,
-                                        _stream_ptr()))
+                                        stream_ptr()))
         return y
 
     def run_static(self, x: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
@@ -135,7 +131,7 @@ class GptOssMoe:
             raise ValueError("run_static needs a CUDA tensor of the operator's io dtype")
         x2 = x.reshape(-1, self.opt.hidden).contiguous()
         y = out if out is not None else torch.empty_like(x2)
-        check(lib().garnet_b200_moe_run_static(self._h, x2.data_ptr(), y.data_ptr(), x2.shape[0], _stream_ptr()))
+        check(lib().garnet_b200_moe_run_static(self._h, x2.data_ptr(), y.data_ptr(), x2.shape[0], stream_ptr()))
         return y
 
     # RunGptOssMoeRoute (gpt_oss_kernels.h:54-56)
@@ -150,7 +146,7 @@ class GptOssMoe:
         ws = torch.empty(need.value, dtype=torch.uint8, device=x.device)
         # the router as `run` evaluates it for this token count
         check(lib().garnet_b200_moe_route_ws(self._h, x2.data_ptr(), selected.data_ptr(), probs.data_ptr(),
-                                             logits.data_ptr(), tokens, ws.data_ptr(), ws.numel(), _stream_ptr()))
+                                             logits.data_ptr(), tokens, ws.data_ptr(), ws.numel(), stream_ptr()))
         return logits, selected, probs
 
     def route_fp32(self, x: torch.Tensor):
@@ -161,7 +157,7 @@ class GptOssMoe:
         selected = torch.empty(tokens, self.opt.top_k, dtype=torch.int32, device=x.device)
         probs = torch.empty(tokens, self.opt.top_k, dtype=torch.float32, device=x.device)
         check(lib().garnet_b200_moe_route(self._h, x2.data_ptr(), selected.data_ptr(), probs.data_ptr(),
-                                          logits.data_ptr(), tokens, _stream_ptr()))
+                                          logits.data_ptr(), tokens, stream_ptr()))
         return logits, selected, probs
 
     def rows_workspace_bytes(self, rows: int) -> int:
@@ -180,7 +176,7 @@ class GptOssMoe:
         ws = workspace if workspace is not None else torch.empty(need, dtype=torch.uint8, device=x2.device)
         ex = row_expert.to(torch.int32).contiguous()
         check(lib().garnet_b200_moe_run_rows(self._h, x2.data_ptr(), ex.data_ptr(), rows, vals.data_ptr(),
-                                             ws.data_ptr(), ws.numel(), _stream_ptr()))
+                                             ws.data_ptr(), ws.numel(), stream_ptr()))
         return vals
 
     def run_rows_hidden(self, rows_x: torch.Tensor, row_expert: torch.Tensor) -> torch.Tensor:
@@ -191,7 +187,7 @@ class GptOssMoe:
         ws = torch.empty(self.rows_workspace_bytes(rows), dtype=torch.uint8, device=x2.device)
         ex = row_expert.to(torch.int32).contiguous()
         check(lib().garnet_b200_moe_run_rows_stage(self._h, 1, x2.data_ptr(), ex.data_ptr(), rows, hid.data_ptr(), None,
-                                                   ws.data_ptr(), ws.numel(), _stream_ptr()))
+                                                   ws.data_ptr(), ws.numel(), stream_ptr()))
         return hid
 
     def run_rows_down(self, hidden: torch.Tensor, row_expert: torch.Tensor) -> torch.Tensor:
@@ -202,7 +198,7 @@ class GptOssMoe:
         ws = torch.empty(self.rows_workspace_bytes(rows), dtype=torch.uint8, device=h2.device)
         ex = row_expert.to(torch.int32).contiguous()
         check(lib().garnet_b200_moe_run_rows_stage(self._h, 2, None, ex.data_ptr(), rows, h2.data_ptr(), vals.data_ptr(),
-                                                   ws.data_ptr(), ws.numel(), _stream_ptr()))
+                                                   ws.data_ptr(), ws.numel(), stream_ptr()))
         return vals
 
     def combine(self, vals: torch.Tensor, probs: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
@@ -210,13 +206,13 @@ class GptOssMoe:
         tokens = probs.shape[0]
         y = out if out is not None else torch.empty(tokens, self.opt.hidden, dtype=self.io_dtype, device=vals.device)
         v, p = vals.contiguous(), probs.contiguous()
-        check(lib().garnet_b200_moe_combine(self._h, v.data_ptr(), p.data_ptr(), y.data_ptr(), tokens, _stream_ptr()))
+        check(lib().garnet_b200_moe_combine(self._h, v.data_ptr(), p.data_ptr(), y.data_ptr(), tokens, stream_ptr()))
         return y
 
     def dequantized(self, which: int, stored_expert: int) -> torch.Tensor:
         rows, cols = (2 * self.inter_local, self.opt.hidden) if which in (0, 2) else (self.opt.hidden, self.inter_local)
         out = torch.empty(rows, cols, dtype=torch.float32, device="cuda")
-        check(lib().garnet_b200_moe_dequant(self._h, which, stored_expert, out.data_ptr(), _stream_ptr()))
+        check(lib().garnet_b200_moe_dequant(self._h, which, stored_expert, out.data_ptr(), stream_ptr()))
         return out
 
     def fault(self) -> int:
@@ -240,7 +236,7 @@ def mxfp4_decode(blocks: torch.Tensor, scales: torch.Tensor) -> torch.Tensor:
     """rows x 32 MXFP4 values -> fp32 (TestGptOssMxfp4Decode)."""
     rows = scales.numel()
     out = torch.empty(rows, 32, dtype=torch.float32, device=blocks.device)
-    check(lib().garnet_b200_mxfp4_decode(blocks.data_ptr(), scales.data_ptr(), out.data_ptr(), rows, _stream_ptr()))
+    check(lib().garnet_b200_mxfp4_decode(blocks.data_ptr(), scales.data_ptr(), out.data_ptr(), rows, stream_ptr()))
     return out
 
 
