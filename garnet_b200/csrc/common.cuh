@@ -82,6 +82,27 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsign
         if (global_timer_ns() - t0 > limit_ns) return false;
     }
 }
+// The same for a warp that shares its scheduler with busy ones: a poll suspends the thread until the phase completes or a
+// time limit passes (10 us here), so that waiting takes no issue slots.
+__device__ __forceinline__ bool mbar_wait_suspended(uint64_t* bar, uint32_t parity, unsigned long long limit_ns = kWaitLimitNs)
+{
+    const auto poll = [&] {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity), "r"(10000)
+            : "memory");
+        return ok != 0;
+    };
+    if (poll()) return true;
+    const unsigned long long t0 = global_timer_ns();
+    while (!poll())
+        if (global_timer_ns() - t0 > limit_ns) return false;
+    return true;
+}
 __device__ __forceinline__ void fence_barrier_init()
 {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");

@@ -4,20 +4,26 @@
 //
 // A CTA owns one kv head and one or two tiles of 128 query rows; a tile's rows are (token, q head of the group), so the
 // K and V rows that a tile stages serve all the q heads of the group, and a causal tile of 16 tokens x 8 heads ends
-// within 16 positions of its last key.  Per 128 keys:
-//   4 loader warps    look up the cache pages and copy 128 K and V rows of 128 bytes (cp.async) into the 128-byte-swizzled
-//                     tile that serves as the K-major operand of Q K^T and as the MN-major operand of P V; a ring of 3;
-//   MMA warp          one thread: P V of the previous keys, then Q K^T of these, tile by tile, so that one tile's MMAs
-//                     run under the other tile's softmax;
-//   2 x 4 softmax     one thread per query row: running maximum (the sink is its first value), p = 2^(s c - m c), the
-//   warps             row's sum in fp32, P back into tensor memory; O in tensor memory is rescaled only when a row's
-//                     maximum has grown by more than 2^8 since the last time (the final division makes that exact).
+// within 16 positions of its last key.  Per 64 keys:
+//   2 loader warps    look up the cache pages and copy 64 K and V rows of 128 bytes (cp.async) into the 128-byte-swizzled
+//                     tile that serves as the K-major operand of Q K^T and as the MN-major operand of P V; a ring of 8,
+//                     whose first 3 steps are requested before the queries are converted;
+//   MMA warp          one thread: P V of these keys when their P is there, then Q K^T of the keys two steps on into the
+//                     columns that P leaves, tile by tile: scores are ready before the softmax wants them;
+//   2 x 4 softmax     one thread per query row: 64 scores into registers, running maximum (the sink is its first value),
+//   warps             p = 2^(s c - m c), the row's sum in fp32, P over the scores in tensor memory; O in tensor memory is
+//                     rescaled only when a row's maximum has grown by more than 2^8 since the last time (the final division
+//                     makes that exact).  The fp32 work runs two values per instruction (f32x2).
 // Numerics: the queries are bf16-valued fp32 (a tile that holds others takes the fp32 row loop instead), so Q K^T has exact
 // products.  P is fp32: it enters the MMA as two bf16 numbers, hi = bf16(p) and lo = bf16(p - hi), which leaves at most
 // 2^-18 p - less than the rounding errors of an fp32 sum over some hundreds of positions, and 2^-9 of the step of the
-// bf16 result.
+// bf16 result.  A row that comes out NaN (infinities in the cache meet a zero piece) is computed again by the row loop.
 //
-// Bound: 16 exponentials per clock and SM, 1024 clocks per tile of 128 x 128 scores, against 768 clocks of MMAs (hi and lo).
+// Bound: per 128 x 64 scores the tensor pipe needs about 460 clocks (8 P V MMAs at 33, 4 Q K^T MMAs at 50) and the exponentials
+// 512 (16 per clock and SM); a pair of tiles takes about 2000 per step, most of it in the instruction issue of the schedulers
+// that a loader or the MMA warp shares with two softmax warps.
+// 2048 tokens, 64 / 8 heads (ncu): 171 us with steps of 128 keys, one set of scores and the next Q K^T behind P V (6050 clocks
+// per 128 keys and pair of tiles, of which the softmax had 2300) -> 119 us.
 #include <algorithm>
 #include <cfloat>
 
@@ -30,20 +36,22 @@ namespace gb200 {
 namespace {
 
 constexpr int kPfRows = 128;          // query rows of a tile (UMMA M, one softmax thread each)
-constexpr int kPfKeys = 128;          // keys of a step (UMMA N of Q K^T, K of P V)
-constexpr int kPfStages = 3;
-constexpr int kPfTileBytes = 128 * 128;
-constexpr int kPfMmaWarp = 8, kPfFirstLoader = 9, kPfLoaders = 4;
+constexpr int kPfKeys = 64;           // keys of a step (UMMA N of Q K^T, K of P V)
+constexpr int kPfStages = 8, kPfAhead = 3;
+constexpr int kPfTileBytes = 128 * 128;          // a tile of queries
+constexpr int kPfKvBytes = kPfKeys * 128;        // a step's K rows, and its V rows
+// 8 softmax warps, MMA, 2 loaders: 11 warps leave a thread 168 registers (13 would leave 128, and the softmax would spill)
+constexpr int kPfMmaWarp = 8, kPfFirstLoader = 9, kPfLoaders = 2;
 constexpr int kPfThreads = (kPfFirstLoader + kPfLoaders) * 32;
-// Tensor memory of a tile: scores (the hi half of P replaces them), the lo half of P, the output.
-constexpr uint32_t kPfColLo = 128, kPfColO = 192, kPfCols = 256;
+// Tensor memory of a tile: two sets of 64 scores (the hi and lo halves of P replace them), the output.
+constexpr uint32_t kPfColLo = 32, kPfColO = 128, kPfCols = 256;
 
 struct PfSmem {
     static constexpr int q = 0;                                    // [2] tiles
     static constexpr int kv = q + 2 * kPfTileBytes;                // [stages] K tile, V tile
-    static constexpr int ok = kv + kPfStages * 2 * kPfTileBytes;   // [stages][4] bits of the keys that exist
-    static constexpr int bars = ok + kPfStages * 16;
-    static constexpr int total = bars + 128 + 1024;                // barriers, and slack for 1024-byte alignment
+    static constexpr int ok = kv + kPfStages * 2 * kPfKvBytes;     // [stages][2] bits of the keys that exist
+    static constexpr int bars = ok + kPfStages * 8;
+    static constexpr int total = bars + 256 + 1024;                // barriers, and slack for 1024-byte alignment
 };
 
 __device__ __forceinline__ float ex2(float x)
@@ -52,14 +60,31 @@ __device__ __forceinline__ float ex2(float x)
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// D[tmem] (+)= A[tmem] * B[smem]; issued by one thread.
-__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, bool accumulate)
+// MMAs whose descriptors arrive as their low words (start address; the high word is the constant of umma_desc_k_sw128): an
+// addition of a constant per MMA.  The issuing thread shares its scheduler with softmax warps, and rebuilding 64-bit
+// descriptors cost it about 100 clocks per MMA, two to three times what the tensor pipe needs for one.
+constexpr uint32_t kPfDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t desc_lo(uint32_t smem_addr) { return ((smem_addr & 0x3FFFFu) >> 4) | (1u << 16); }
+// D[tmem] (+)= A[smem] * B[smem]
+__device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, bool accumulate)
 {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+        "mov.b64 a, {%1, %5};\n\tmov.b64 b, {%2, %5};\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(uint32_t(accumulate))
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t}" ::"r"(d_tmem),
+        "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(uint32_t(accumulate)), "n"(kPfDescHi)
+        : "memory");
+}
+// D[tmem] (+)= A[tmem] * B[smem]
+__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc, bool accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\t"
+        "mov.b64 b, {%2, %5};\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n\t}" ::"r"(d_tmem),
+        "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(uint32_t(accumulate)), "n"(kPfDescHi)
         : "memory");
 }
 __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16])
@@ -69,6 +94,32 @@ __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r
         "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
         "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
         : "memory");
+}
+__device__ __forceinline__ float max3(float a, float b, float c)
+{
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+// Two fp32 values per instruction.
+__device__ __forceinline__ uint64_t f32x2(float lo, float hi)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void f32x2_split(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
@@ -80,7 +131,8 @@ __device__ __forceinline__ uint32_t bit_range(int lo, int hi)
     return (hi == 32 ? 0xffffffffu : (1u << hi) - 1u) & ~((1u << lo) - 1u);
 }
 
-__global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(const OssAttn p, const int qtiles)
+template <int qtiles>
+__global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(const OssAttn p)
 {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -89,22 +141,43 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
     uint32_t* ok_bits = reinterpret_cast<uint32_t*>(smem + PfSmem::ok);
     uint64_t* kv_full = reinterpret_cast<uint64_t*>(smem + PfSmem::bars);   // [stages]
     uint64_t* kv_empty = kv_full + kPfStages;                               // [stages]
-    uint64_t* s_full = kv_empty + kPfStages;                                // [2] scores written (and the P V before them done)
-    uint64_t* p_full = s_full + 2;                                          // [2] P written
-    uint64_t* o_full = p_full + 2;                                          // [2] last P V done
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
+    uint64_t* s_full = kv_empty + kPfStages;                                // [2 tiles][2 sets] scores written
+    uint64_t* p_full = s_full + 4;                                          // [2 tiles][2 sets] P written
+    uint64_t* o_full = p_full + 4;                                          // [2 tiles] P V of a step done
+    uint64_t* o_done = o_full + 2;                                          // [2 tiles] the last P V done
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int kv = blockIdx.x, b = blockIdx.z, group = p.q_heads / p.kv_heads;
     const int tile_tokens = kPfRows / group;   // the launch makes sure of group <= 128
     // the tiles with the most keys first, so that the short ones fill the gaps at the end
     const int t0 = int(gridDim.y - 1 - blockIdx.y) * tile_tokens * qtiles, t1 = min(p.tokens, t0 + tile_tokens * qtiles);
     const int limit = p.logical_pages * p.page_size;
-    const int start = p.starts[b];
-    const bool active = p.active[b] != 0;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kPfStages; ++s) {
+            mbar_init(&kv_full[s], kPfLoaders);
+            mbar_init(&kv_empty[s], 1);
+        }
+        for (int s = 0; s < 4; ++s) {
+            mbar_init(&s_full[s], 1);
+            mbar_init(&p_full[s], 4);
+            if (s < 2) mbar_init(&o_full[s], 1), mbar_init(&o_done[s], 1);
+        }
+        *abort_flag = 0;
+        fence_barrier_init();
+    }
+    const uint32_t tmem_cols = kPfCols * qtiles;
+    if (warp == kPfMmaWarp) {
+        tmem_alloc(tmem_slot, tmem_cols);
+        tmem_relinquish();
+    }
+    pdl_wait();   // the cache rows and the queries come from the kernels before this one
 
     // keys that some row of the CTA sees
+    const int start = p.starts[b];
+    const bool active = p.active[b] != 0;
     int first_end, last_end;
     if (p.prefill) first_end = max(1, start + t0 + 1), last_end = min(limit, start + t1);
     else first_end = last_end = p.lengths[b];
@@ -112,132 +185,133 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
     const int key0 = p.window ? max(0, first_end - p.window) : 0, key1 = last_end;
     const int steps = (key1 - key0 + kPfKeys - 1) / kPfKeys;
 
-    // ---- queries: fp32 to bf16, 128-byte-swizzled K-major tiles
-    const int packed = (p.q_heads + 2 * p.kv_heads) * kOssDim;
-    int inexact = 0;
-    for (int i = threadIdx.x; i < qtiles * kPfRows * 8; i += kPfThreads) {
-        const int row = i >> 3, piece = i & 7, r = row & (kPfRows - 1), in_tile = r / group;
-        const int t = t0 + (row >> 7) * tile_tokens + in_tile, head = kv * group + r % group;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (steps && in_tile < tile_tokens && t < t1) {
-            const float4* src = reinterpret_cast<const float4*>(p.qkv + (size_t(b) * p.tokens + t) * packed + head * kOssDim + piece * 8);
-            const float4 f0 = __ldg(src), f1 = __ldg(src + 1);
-            const float f[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
-#pragma unroll
-            for (int j = 0; j < 8; ++j) inexact |= int(__float_as_uint(f[j]) & 0xffffu);
-            v = make_uint4(bf16x2_of(f0.x, f0.y), bf16x2_of(f0.z, f0.w), bf16x2_of(f1.x, f1.y), bf16x2_of(f1.z, f1.w));
-        }
-        *reinterpret_cast<uint4*>(q_tiles + row * 128 + ((piece ^ (row & 7)) << 4)) = v;
-    }
-    fence_proxy_async_smem();
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < kPfStages; ++s) {
-            mbar_init(&kv_full[s], kPfLoaders);
-            mbar_init(&kv_empty[s], 1);
-        }
-        for (int s = 0; s < 2; ++s) {
-            mbar_init(&s_full[s], 1);
-            mbar_init(&p_full[s], 4);
-            mbar_init(&o_full[s], 1);
-        }
-        *abort_flag = 0;
-        fence_barrier_init();
-    }
-    if (__syncthreads_or(inexact) || steps == 0) {
-        // queries that are not bf16 values (outside the operand's contract), or no visible key at all
-        const int rows = (t1 - t0) * group;
-        for (int i = warp; i < rows; i += kPfThreads / 32)
-            oss_attention_row(p, b * p.tokens + t0 + i / group, kv * group + i % group, lane);
-        return;
-    }
-    const uint32_t tmem_cols = kPfCols * qtiles;
-    if (warp == kPfMmaWarp) {
-        tmem_alloc(tmem_slot, tmem_cols);
-        tmem_relinquish();
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
-
-    if (warp >= kPfFirstLoader) {
-        // -------------------------------------------------------------- loaders
-        const int lw = warp - kPfFirstLoader;
-        for (int j = 0; j < steps && !*abort_flag; ++j) {
-            const int st = j % kPfStages;
-            if (j >= kPfStages && !mbar_wait_bounded(&kv_empty[st], ((j / kPfStages) - 1) & 1)) {
-                *abort_flag = 1;
-                break;
-            }
-            const int pos = key0 + j * kPfKeys + lw * 32 + lane;
-            const size_t off = pos < key1 ? oss_cache_offset(p, b, pos, kv) : SIZE_MAX;
+    // ---- loaders: the row of a key (one per lane), and the copies of a step
+    const int lw = warp - kPfFirstLoader;
+    const auto look_up = [&](int j) -> unsigned long long {
+        const int pos = key0 + j * kPfKeys + lw * 32 + lane;
+        return pos < key1 ? oss_cache_offset(p, b, pos, kv) : SIZE_MAX;
+    };
+    const auto request = [&](int j, unsigned long long off) {
+        if (j < steps) {
+            const int st = j % kPfStages, piece = lane & 7;
             const uint32_t exists = __ballot_sync(0xffffffffu, off != SIZE_MAX);
-            if (lane == 0) ok_bits[st * 4 + lw] = exists;
-            const uint32_t kt = smem_u32(kv_ring + st * 2 * kPfTileBytes) + lw * 32 * 128, vt = kt + kPfTileBytes;
-            const int piece = lane & 7;
+            if (lane == 0) ok_bits[st * 2 + lw] = exists;
+            const uint32_t kt = smem_u32(kv_ring + st * 2 * kPfKvBytes) + lw * 32 * 128, vt = kt + kPfKvBytes;
 #pragma unroll
             for (int it = 0; it < 8; ++it) {
                 const int row = it * 4 + (lane >> 3);
-                const unsigned long long o = __shfl_sync(0xffffffffu, static_cast<unsigned long long>(off), row);
+                const unsigned long long o = __shfl_sync(0xffffffffu, off, row);
                 const bool valid = o != SIZE_MAX;   // rows that do not exist are filled with zeros
                 const size_t at = (valid ? o : 0) + piece * 8;
                 const uint32_t to = row * 128 + ((piece ^ (row & 7)) << 4);
                 cp_async16(kt + to, p.keys + at, valid);
                 cp_async16(vt + to, p.values + at, valid);
             }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            if (j > 0) {
-                asm volatile("cp.async.wait_group 1;" ::: "memory");
-                fence_proxy_async_smem();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&kv_full[(j - 1) % kPfStages]);
-            }
         }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    unsigned long long ahead = SIZE_MAX;   // rows of the next step to request
+    int inexact = 0;
+    if (warp >= kPfFirstLoader) {
+        const unsigned long long first[kPfAhead] = {look_up(0), look_up(1), look_up(2)};
+#pragma unroll
+        for (int j = 0; j < kPfAhead; ++j) request(j, first[j]);
+        ahead = look_up(kPfAhead);
+    } else {
+        // ---- queries: fp32 to bf16, 128-byte-swizzled K-major tiles
+        const int packed = (p.q_heads + 2 * p.kv_heads) * kOssDim;
+#pragma unroll 4
+        for (int i = threadIdx.x; i < qtiles * kPfRows * 8; i += kPfFirstLoader * 32) {
+            const int row = i >> 3, piece = i & 7, r = row & (kPfRows - 1), in_tile = r / group;
+            const int t = t0 + (row >> 7) * tile_tokens + in_tile, head = kv * group + r % group;
+            uint4 v = make_uint4(0, 0, 0, 0);
+            if (steps && in_tile < tile_tokens && t < t1) {
+                const float4* src = reinterpret_cast<const float4*>(p.qkv + (size_t(b) * p.tokens + t) * packed + head * kOssDim + piece * 8);
+                const float4 f0 = __ldg(src), f1 = __ldg(src + 1);
+                const float f[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
+#pragma unroll
+                for (int j = 0; j < 8; ++j) inexact |= int(__float_as_uint(f[j]) & 0xffffu);
+                v = make_uint4(bf16x2_of(f0.x, f0.y), bf16x2_of(f0.z, f0.w), bf16x2_of(f1.x, f1.y), bf16x2_of(f1.z, f1.w));
+            }
+            *reinterpret_cast<uint4*>(q_tiles + row * 128 + ((piece ^ (row & 7)) << 4)) = v;
+        }
         fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0 && !*abort_flag) mbar_arrive(&kv_full[(steps - 1) % kPfStages]);
+    }
+    tc_fence_before();
+    const bool row_loop = __syncthreads_or(inexact) || steps == 0;
+    tc_fence_after();
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    if (row_loop) {
+        // queries that are not bf16 values (outside the operand's contract), or no visible key at all
+        const int rows = (t1 - t0) * group;
+        for (int i = warp; i < rows; i += kPfThreads / 32)
+            oss_attention_row(p, b * p.tokens + t0 + i / group, kv * group + i % group, lane);
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        if (warp == kPfMmaWarp) tmem_dealloc(tmem_base, tmem_cols);
+        return;
+    }
+
+    if (warp >= kPfFirstLoader) {
+        // -------------------------------------------------------------- loaders
+        // a step is announced as soon as it is there, before the wait for the stage of the next request
+        for (int j = 0; j < steps && !*abort_flag; ++j) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kPfAhead - 1) : "memory");
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&kv_full[j % kPfStages]);
+            const int next = j + kPfAhead;
+            if (next >= kPfStages && next < steps && !mbar_wait_suspended(&kv_empty[next % kPfStages], ((next / kPfStages) - 1) & 1)) {
+                *abort_flag = 1;
+                break;
+            }
+            request(next, ahead);
+            ahead = look_up(next + 1);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
     } else if (warp == kPfMmaWarp) {
         // ----------------------------------------------------------- MMA issuer
-        if (lane == 0) {
-            const uint32_t idesc_qk = umma_idesc_f16(1, kPfRows, kPfKeys);
-            const uint32_t idesc_pv = umma_idesc_f16(1, kPfRows, kOssDim) | (1u << 16);   // V: MN-major
-            for (int j = 0; j <= steps && !*abort_flag; ++j) {
-                const int st = j % kPfStages;
-                if (j < steps && !mbar_wait_bounded(&kv_full[st], (j / kPfStages) & 1)) {
-                    *abort_flag = 1;
-                    break;
-                }
-                for (int q = 0; q < qtiles; ++q) {
-                    const uint32_t tm = tmem_base + q * kPfCols;
-                    if (j > 0) {
-                        if (!mbar_wait_bounded(&p_full[q], (j - 1) & 1)) {
-                            *abort_flag = 1;
-                            break;
-                        }
-                        tc_fence_after();
-                        const uint32_t v_addr = smem_u32(kv_ring + ((j - 1) % kPfStages) * 2 * kPfTileBytes) + kPfTileBytes;
+        if (elect_one()) {
+            constexpr uint32_t idesc_qk = umma_idesc_f16(1, kPfRows, kPfKeys);
+            constexpr uint32_t idesc_pv = umma_idesc_f16(1, kPfRows, kOssDim) | (1u << 16);   // V: MN-major
+            const uint32_t q_lo = desc_lo(smem_u32(q_tiles)), k_lo = desc_lo(smem_u32(kv_ring)), v_lo = desc_lo(smem_u32(kv_ring + kPfKvBytes));
+            constexpr uint32_t kStage = 2 * kPfKvBytes >> 4;
+            // scores of step j of tile q, into set j & 1
+            const auto scores = [&](int j, int q) {
+                const uint32_t d = tmem_base + q * kPfCols + (j & 1) * kPfKeys;
+                const uint32_t a = q_lo + q * (kPfTileBytes >> 4), k = k_lo + (j % kPfStages) * kStage;
 #pragma unroll
-                        for (int half = 0; half < 2; ++half)
+                for (int k16 = 0; k16 < kOssDim / 16; ++k16) umma_ss(d, a + k16 * 2, k + k16 * 2, idesc_qk, k16 > 0);
+                umma_commit(&s_full[q * 2 + (j & 1)]);
+            };
+            bool good = true;
+            for (int j = 0; j < 2 && j < steps && good; ++j) {
+                good = mbar_wait_suspended(&kv_full[j], 0);
+                tc_fence_after();
 #pragma unroll
-                            for (int k16 = 0; k16 < kPfKeys / 16; ++k16)
-                                umma_f16_ts(tm + kPfColO, tm + half * kPfColLo + k16 * 8, umma_desc_k_sw128(v_addr + k16 * 2048), idesc_pv,
-                                            j > 1 || half > 0 || k16 > 0);
-                    }
-                    if (j < steps) {
-                        tc_fence_after();
-                        const uint32_t q_addr = smem_u32(q_tiles + q * kPfTileBytes), k_addr = smem_u32(kv_ring + st * 2 * kPfTileBytes);
-#pragma unroll
-                        for (int k16 = 0; k16 < kOssDim / 16; ++k16)
-                            umma_f16(tm, umma_desc_k_sw128(q_addr + k16 * 32), umma_desc_k_sw128(k_addr + k16 * 32), idesc_qk, k16 > 0);
-                        umma_commit(&s_full[q]);
-                    } else {
-                        umma_commit(&o_full[q]);
-                    }
-                }
-                if (j > 0) umma_commit(&kv_empty[(j - 1) % kPfStages]);
+                for (int q = 0; q < qtiles; ++q) scores(j, q);
             }
+            for (int j = 0; j < steps && good; ++j) {
+                const uint32_t v = v_lo + (j % kPfStages) * kStage;
+#pragma unroll
+                for (int q = 0; q < qtiles; ++q) {
+                    good = good && mbar_wait_suspended(&p_full[q * 2 + (j & 1)], (j >> 1) & 1);
+                    if (good && q == 0 && j + 2 < steps) good = mbar_wait_suspended(&kv_full[(j + 2) % kPfStages], ((j + 2) / kPfStages) & 1);
+                    if (!good) break;
+                    tc_fence_after();
+                    const uint32_t d = tmem_base + q * kPfCols + kPfColO, a = tmem_base + q * kPfCols + (j & 1) * kPfKeys;
+#pragma unroll
+                    for (int half = 0; half < 2; ++half)
+#pragma unroll
+                        for (int k16 = 0; k16 < kPfKeys / 16; ++k16)
+                            umma_ts(d, a + half * kPfColLo + k16 * 8, v + k16 * (2048 >> 4), idesc_pv, j > 0 || half > 0 || k16 > 0);
+                    umma_commit(j + 1 < steps ? &o_full[q] : &o_done[q]);
+                    if (j + 2 < steps) scores(j + 2, q);
+                }
+                umma_commit(&kv_empty[j % kPfStages]);
+            }
+            if (!good) *abort_flag = 1;
         }
+        __syncwarp();
     } else if ((warp >> 2) < qtiles) {
         // -------------------------------------------------------------- softmax
         const int q = warp >> 2, r = (warp & 3) * 32 + lane;
@@ -253,41 +327,39 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
         float sum = 1.f;                                       // the sink's own term
         for (int j = 0; j < steps && !*abort_flag; ++j) {
             const int st = j % kPfStages, kb = key0 + j * kPfKeys;
-            if (!mbar_wait_bounded(&kv_full[st], (j / kPfStages) & 1) || !mbar_wait_bounded(&s_full[q], j & 1)) {
+            const uint32_t ts = tm + (j & 1) * kPfKeys;
+            if (!mbar_wait_suspended(&kv_full[st], (j / kPfStages) & 1) || !mbar_wait_suspended(&s_full[q * 2 + (j & 1)], (j >> 1) & 1)) {
                 *abort_flag = 1;
                 break;
             }
             tc_fence_after();
-            uint32_t vis[4];
-            bool all = true;
+            uint32_t s[2][32];
+            tmem_ld_32x32(ts, s[0]);
+            tmem_ld_32x32(ts + 32, s[1]);
+            const uint32_t there[2] = {ok_bits[st * 2], ok_bits[st * 2 + 1]};
+            tmem_ld_wait();
+            if (!__all_sync(0xffffffffu, begin <= kb && end >= kb + kPfKeys && (there[0] & there[1]) == 0xffffffffu)) {
 #pragma unroll
-            for (int w = 0; w < 4; ++w) {
-                vis[w] = ok_bits[st * 4 + w] & bit_range(begin - kb - 32 * w, end - kb - 32 * w);
-                all = all && vis[w] == 0xffffffffu;
-            }
-            all = __all_sync(0xffffffffu, all);
-            float top = -INFINITY;
+                for (int w = 0; w < 2; ++w) {
+                    const uint32_t vis = there[w] & bit_range(begin - kb - 32 * w, end - kb - 32 * w);
 #pragma unroll
-            for (int w = 0; w < 4; ++w) {
-                uint32_t s[32];
-                tmem_ld_32x32(tm + 32 * w, s);
-                tmem_ld_wait();
-                if (all) {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) top = fmaxf(top, __uint_as_float(s[i]));
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) top = fmaxf(top, (vis[w] >> i) & 1 ? __uint_as_float(s[i]) : -INFINITY);
+                    for (int i = 0; i < 32; ++i) s[w][i] = (vis >> i) & 1 ? s[w][i] : 0xff800000u;   // -inf
                 }
             }
-            top *= c;
+            float m[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+            for (int i = 0; i < 32; ++i) m[i & 3] = max3(m[i & 3], __uint_as_float(s[0][i]), __uint_as_float(s[1][i]));
+            const float top = fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3])) * c;
             const bool grow = j == 0 ? top > ref : top > ref + 8.f;
             if (__any_sync(0xffffffffu, grow)) {
                 const float f = grow ? ex2(ref - top) : 1.f;
                 if (grow) ref = top;
                 sum *= f;
                 if (j > 0) {
-#pragma unroll
+                    // P V of the step before has to be in O (P V of step j - 2 was done before these scores)
+                    if (!mbar_wait_suspended(&o_full[q], (j - 1) & 1)) *abort_flag = 1;
+                    tc_fence_after();
+#pragma unroll 1
                     for (int h = 0; h < 4; ++h) {
                         uint32_t o[16];
                         tmem_ld_32x16(tm + kPfColO + 16 * h, o);
@@ -299,38 +371,40 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
                 }
             }
             const float base = ref == -INFINITY ? 0.f : ref;
-            float part[2] = {0.f, 0.f};
+            const uint64_t scale2 = f32x2(c, c), base2 = f32x2(-base, -base), minus1 = f32x2(-1.f, -1.f);
+            uint64_t part2[2] = {0, 0};
 #pragma unroll
-            for (int w = 0; w < 4; ++w) {
-                uint32_t s[32], hi[16], lo[16];
-                tmem_ld_32x32(tm + 32 * w, s);
-                tmem_ld_wait();
+            for (int w = 0; w < 2; ++w) {
+                uint32_t hi[16], lo[16];
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                    float a = ex2(fmaf(__uint_as_float(s[2 * i]), c, -base)), d = ex2(fmaf(__uint_as_float(s[2 * i + 1]), c, -base));
-                    if (!all) {
-                        a = (vis[w] >> (2 * i)) & 1 ? a : 0.f;
-                        d = (vis[w] >> (2 * i + 1)) & 1 ? d : 0.f;
-                    }
-                    part[0] += a;
-                    part[1] += d;
+                    float a, d;
+                    f32x2_split(fma2(f32x2(__uint_as_float(s[w][2 * i]), __uint_as_float(s[w][2 * i + 1])), scale2, base2), a, d);
+                    a = ex2(a), d = ex2(d);
+                    const uint64_t e2 = f32x2(a, d);
+                    part2[i & 1] = add2(part2[i & 1], e2);
                     hi[i] = bf16x2_of(a, d);
-                    lo[i] = bf16x2_of(a - __uint_as_float(hi[i] << 16), d - __uint_as_float(hi[i] & 0xffff0000u));
+                    float la, ld;
+                    f32x2_split(fma2(f32x2(__uint_as_float(hi[i] << 16), __uint_as_float(hi[i] & 0xffff0000u)), minus1, e2), la, ld);
+                    lo[i] = bf16x2_of(la, ld);
                 }
-                tmem_st_32x16(tm + 16 * w, hi);
-                tmem_st_32x16(tm + kPfColLo + 16 * w, lo);
+                tmem_st_32x16(ts + 16 * w, hi);
+                tmem_st_32x16(ts + kPfColLo + 16 * w, lo);
             }
+            float part[2];
+            f32x2_split(add2(part2[0], part2[1]), part[0], part[1]);
             sum += part[0] + part[1];
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&p_full[q]);
+            if (lane == 0) mbar_arrive(&p_full[q * 2 + (j & 1)]);
         }
-        if (!*abort_flag && !mbar_wait_bounded(&o_full[q], 0)) *abort_flag = 1;
+        if (!*abort_flag && !mbar_wait_suspended(&o_done[q], 0)) *abort_flag = 1;
         tc_fence_after();
         // a wait that gave up leaves NaNs, which no caller can take for a result
         if (*abort_flag) sum = NAN;
         float* out = p.out + (size_t(b) * p.tokens + t) * p.q_heads * kOssDim + head * kOssDim;
+        bool bad = false;
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
             uint32_t o[16];
@@ -341,11 +415,18 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
                 for (int i = 0; i < 4; ++i) {
                     float v[4];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) v[e] = end > begin ? bf16_round_f(__uint_as_float(o[4 * i + e]) / sum) : 0.f;
+                    for (int e = 0; e < 4; ++e) {
+                        v[e] = end > begin ? bf16_round_f(__uint_as_float(o[4 * i + e]) / sum) : 0.f;
+                        bad = bad || isnan(v[e]);
+                    }
                     *reinterpret_cast<float4*>(out + 16 * h + 4 * i) = make_float4(v[0], v[1], v[2], v[3]);
                 }
             }
             __syncwarp();
+        }
+        for (uint32_t redo = __ballot_sync(0xffffffffu, bad && !*abort_flag); redo; redo &= redo - 1) {
+            const int from = __ffs(redo) - 1;
+            oss_attention_row(p, __shfl_sync(0xffffffffu, b * p.tokens + t, from), __shfl_sync(0xffffffffu, head, from), lane);
         }
     }
     tc_fence_before();
@@ -373,10 +454,19 @@ int oss_prefill_launch(const OssAttn& p, cudaStream_t stream)
     // Two tiles per CTA keep the exponential unit busy while the other tile's MMAs run; with fewer CTAs than SMs one tile each
     // uses twice the SMs.
     const int qtiles = (long long)p.batch * p.kv_heads * blocks(2) >= kSmCount ? 2 : 1;
-    GB_CUDA(cudaFuncSetAttribute(oss_attention_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PfSmem::total));
-    oss_attention_prefill_kernel<<<dim3(unsigned(p.kv_heads), unsigned(blocks(qtiles)), unsigned(p.batch)), kPfThreads, PfSmem::total,
-                                   stream>>>(p, qtiles);
-    GB_CUDA(cudaGetLastError());
+    const auto kernel = qtiles == 2 ? oss_attention_prefill_kernel<2> : oss_attention_prefill_kernel<1>;
+    GB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PfSmem::total));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(p.kv_heads), unsigned(blocks(qtiles)), unsigned(p.batch));
+    cfg.blockDim = dim3(kPfThreads);
+    cfg.dynamicSmemBytes = PfSmem::total;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    GB_CUDA(cudaLaunchKernelEx(&cfg, kernel, p));
     return GARNET_B200_OK;
 }
 

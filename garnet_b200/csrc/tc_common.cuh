@@ -89,7 +89,7 @@ __device__ __forceinline__ uint64_t umma_desc_k_sw128(uint32_t smem_addr)
 
 // Instruction descriptor for kind::f16: fp32 accumulate, A and B K-major.
 // fmt: 0 = fp16, 1 = bf16.
-__host__ __device__ inline uint32_t umma_idesc_f16(int fmt, int m, int n)
+__host__ __device__ constexpr uint32_t umma_idesc_f16(int fmt, int m, int n)
 {
     return (1u << 4) | (uint32_t(fmt) << 7) | (uint32_t(fmt) << 10) | (uint32_t(n >> 3) << 17) | (uint32_t(m >> 4) << 24);
 }

@@ -123,3 +123,15 @@ def test_rows_that_see_the_whole_sequence():
 
 def test_queries_that_are_not_bf16_values():
     check(make(20, [50], 0, exact=False, seed=4))
+
+
+def test_infinite_values_stay_infinite():
+    c = make(40, [300], 0, seed=5)
+    slot = c["table"][0, 3]
+    c["values"][1, slot, 2, 0, 7] = math.inf
+    c["values"][1, slot, 5, 1, 9] = -math.inf
+    got, (w, _) = run(c).to(D).reshape(40, 64, 64), want(c)
+    w = w.reshape(40, 64, 64)
+    assert bool((got[:, :8, 7] == math.inf).all()) and bool((got[:, 8:16, 9] == -math.inf).all())
+    rest = torch.isfinite(w)
+    assert torch.equal(torch.isfinite(got), rest) and float((got - w)[rest].abs().max()) < 2e-2
