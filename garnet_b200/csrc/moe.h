@@ -86,8 +86,8 @@ struct Moe {
     struct alignas(64) TensorMapStorage { unsigned char bytes[128]; };
     int mx_kp[2] = {0, 0}, mx_kslabs[2] = {0, 0};   // block-scaled path: K padded to 128, and in slabs of 128
     bool mx_ok = false;
-    struct QMapCache {                 // TMA view of the quantised rows of the last call
-        TensorMapStorage map;
+    struct QMapCache {                 // TMA views of the quantised rows of the last call, by rows of the box (moe_mx.cu)
+        TensorMapStorage maps[3];
         const void* base = nullptr;
         int kp = 0, q_rows = 0;
     };
@@ -122,8 +122,7 @@ struct Moe {
     int init_mxr(int pass, const uint8_t* blocks, const uint8_t* scales, int first_stored, int count, cudaStream_t stream);
     int finish_mxr();
     int dequant_block_scaled(int pass, int stored_expert, float* out, cudaStream_t stream);
-    int launch_mxr_gemm(bool up, const MoeWorkspacePtrs& w, const void* q_map, int q_rows, int tiles_max,
-                        cudaStream_t stream);
+    int launch_mxr_gemm(bool up, const MoeWorkspacePtrs& w, const QMapCache& q, int tiles_max, cudaStream_t stream);
     int launch_mx(bool up, const MoeWorkspacePtrs& w, const void* x, int x_is_sorted, int tokens, int slots, int topk,
                   cudaStream_t stream);
     // The block-scaled path pays off once experts get several rows each (measured

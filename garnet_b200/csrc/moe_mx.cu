@@ -170,6 +170,7 @@ __global__ void mx_quant_rows_kernel(const T* __restrict__ src, const int* __res
     const int e = s_expert;
     const int idx = pos - offsets[e];
     const int tile = tile_prefix[e] + idx / nt, r = idx % nt;
+    const int box = mx_tile_box(min(nt, offsets[e + 1] - offsets[e] - idx / nt * nt));
     const T* row = src + size_t(sorted ? sorted[pos] / div : pos) * k;
     const int kslabs = kp / kMxSlab;
     for (int b = threadIdx.x; b < kp / 32; b += blockDim.x) {
@@ -197,6 +198,10 @@ __global__ void mx_quant_rows_kernel(const T* __restrict__ src, const int* __res
         // both pieces of the row carry the same scale: one byte of the tile's scale atom
         uint8_t* atom = sf + (size_t(tile) * kslabs + (b >> 2)) * kMxAtom;
         atom[(r & 31) * 16 + ((r >> 5) & 3) * 4 + (b & 3)] = uint8_t(sbyte);
+        if (box != kMxBoxFull) {   // the pieces of a small tile are one operand, which reads a scale for each
+            const int r2 = r + box;
+            atom[(r2 & 31) * 16 + ((r2 >> 5) & 3) * 4 + (b & 3)] = uint8_t(sbyte);
+        }
     }
 }
 
@@ -298,15 +303,19 @@ int Moe::launch_mx(bool up, const MoeWorkspacePtrs& w, const void* x, int x_is_s
     if (c.base != w.mx_q || c.kp != kp || c.q_rows != plan.q_rows) {
         const cuuint64_t dims[2] = {cuuint64_t(kp), cuuint64_t(2) * plan.q_rows};
         const cuuint64_t strides[1] = {cuuint64_t(kp)};
-        const cuuint32_t box[2] = {kMxSlab, cuuint32_t(nt)};
-        if (int rc = mx_encode_tensor_map(reinterpret_cast<CUtensorMap*>(&c.map), CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, w.mx_q, dims,
-                                          strides, box, CU_TENSOR_MAP_SWIZZLE_128B))
-            return rc;
+        const int rows[3] = {kMxBoxFull, kMxBoxSmall, kMxBoxMid};
+        c.base = nullptr;
+        for (int i = 0; i < 3; ++i) {
+            const cuuint32_t box[2] = {kMxSlab, cuuint32_t(rows[i])};
+            if (int rc = mx_encode_tensor_map(reinterpret_cast<CUtensorMap*>(&c.maps[i]), CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, w.mx_q,
+                                              dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B))
+                return rc;
+        }
         c.base = w.mx_q;
         c.kp = kp;
         c.q_rows = plan.q_rows;
     }
-    return launch_mxr_gemm(up, w, &c.map, plan.q_rows, plan.tiles_max, stream);
+    return launch_mxr_gemm(up, w, c, plan.tiles_max, stream);
 }
 
 }  // namespace gb200

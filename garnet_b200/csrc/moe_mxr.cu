@@ -1,11 +1,13 @@
-// Block-scaled grouped GEMM of the gpt-oss MXFP4 experts with the routed rows as the
-// UMMA M operand and 240 weight rows as the N operand.
+// Block-scaled grouped GEMM of the gpt-oss MXFP4 experts, in two orientations.
 //
-// Why this orientation.  A tcgen05.mma of kind::mxf8f6f4 with M = 128, K = 32 keeps the
-// tensor pipe busy for about 130 cycles whatever its N (the time to stream its 128 x
-// 32-byte A tile), and an N near 256 has that much math.  With the weights as A and a
-// tile's rows as N (moe_mx.cu) an expert with 130 rows runs at half the pipe's rate;
-// here every MMA is 240 wide, and what a partly filled row tile wastes is M, not N.
+// Tiles of 57-128 routed rows: the rows are the UMMA M operand and 240 weight rows the N operand.  A tcgen05.mma of kind
+// mxf8f6f4 with M = 128, K = 32 takes 122 clocks at N = 240, 66 at N = 128, 50 at N = 64 and 41 at N = 32 in either operand
+// order (measured alone), so what a partly filled row tile wastes is M.
+// Tiles of at most 56 rows - the last rows of an expert, and most tiles of a short or skewed prompt - the other way round:
+// the weight rows are M (two blocks of 128, the last 16 rows of the second are not used) and both pieces of the activation
+// rows are one N operand, first pieces then second pieces: N = 64 for up to 32 rows, 112 for up to 56 (what fits twice
+// beside each other in an accumulator).  Per 240 weight rows and 32 columns 100 or 124 clocks instead of 244, and 8 or 14 KiB
+// of activations per stage instead of 32.
 // 240 = the widest N for which two accumulators (2 x 240 columns) and the scale copies
 // (4 + 8 columns) fit the 512 columns of tensor memory; it divides the gpt-oss
 // matrices (5760 = 24 x 240, 2880 = 12 x 240).
@@ -22,9 +24,10 @@
 //      read 85 bytes per cycle of the 128 the SM has); their e8m0 scales as two
 //      512-byte atoms;
 //   D  fp32 in tensor memory, lane = routed row, column = weight row, double-buffered.
-// Each K block of 32 takes two MMAs (first piece, second piece) into the same D.
+// Each K block of 32 takes two MMAs: first piece and second piece into the same D, or first and second block of weight rows.
 // Epilogue: a thread owns one routed row: gate and up of a channel are neighbouring
-// columns, outputs leave as 16-byte stores.
+// columns, outputs leave as 16-byte stores.  In the small tiles it owns one weight row: the pieces' columns are added, gate
+// and up of a channel are neighbouring lanes, which exchange every other column.
 #include <algorithm>
 
 #include "layout.h"
@@ -36,7 +39,9 @@ namespace gb200 {
 
 constexpr int kRxRows = 128;          // routed rows per tile (UMMA M)
 constexpr int kRxN = kMxBlockRows;    // weight rows per tile (UMMA N): 240
-constexpr int kRxEpiWarps = 8;
+// 16 epilogue warps, four per scheduler: their chains (accumulator -> bias -> roundings -> exponential -> division) are long,
+// and with two per scheduler the epilogue of a full gate/up tile took 31k clocks while its MMAs take 22k.
+constexpr int kRxEpiWarps = 16, kRxEpiGroups = kRxEpiWarps / 4;
 constexpr int kRxFirstEpi = 3;                          // warp 0: producer, warp 1: MMA issuer, warp 2: spare
 constexpr int kRxThreads = (kRxFirstEpi + kRxEpiWarps) * 32;
 constexpr int kRxPkBytes = kMxBlockBytes;               // 15360: packed weight block of a stage
@@ -76,6 +81,7 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes
 
 struct RxItem {
     int expert, tile, ntile, rows, row0;
+    int box;   // rows that a TMA of the tile brings: 32, 56 (weights as M) or 128
 };
 __device__ __forceinline__ RxItem rx_decode(const RxParams& p, const int* tile_prefix, int item, int& cursor)
 {
@@ -87,13 +93,64 @@ __device__ __forceinline__ RxItem rx_decode(const RxParams& p, const int* tile_p
     it.ntile = item % p.ntiles;
     it.row0 = p.offsets[cursor] + (t - tile_prefix[cursor]) * kRxRows;
     it.rows = min(kRxRows, p.offsets[cursor + 1] - it.row0);
+    it.box = mx_tile_box(it.rows);
     return it;
+}
+
+// bf16(sigmoid-gated unit) of a channel, with the reference's rounding points.
+__device__ __forceinline__ uint32_t rx_swiglu_f16(float gate, float up, float limit)
+{
+    gate = fminf(gate, limit);
+    up = fminf(limit, fmaxf(-limit, up));
+    const float sig = bf16_round_f(1.f / (1.f + expf(-bf16_round_f(1.702f * gate))));
+    const float glu = bf16_round_f(gate * sig);
+    return __half_as_ushort(__float2half_rn(bf16_round_f(glu * bf16_round_f(up + 1.f))));
+}
+
+// A tile of at most 56 rows: the calling thread owns weight row `n` of the block, column c of the accumulator is the first
+// piece of routed row c and column box + c the second; groups of 8 columns from `first` on, every other one.
+template <bool kUp>
+__device__ __forceinline__ void rx_small_epilogue(const RxParams& p, const RxItem& it, const float* bias, uint32_t taddr, int n, int first, int lane)
+{
+    const int row = it.ntile * kRxN + n;
+    const bool live = n < kRxN && row < p.rows;
+    const float b = live ? bias[row] : 0.f;
+    for (int c0 = first; c0 < it.rows; c0 += 16) {
+        uint32_t hi[8], lo[8];
+        tmem_ld_32x8(taddr + c0, hi);
+        tmem_ld_32x8(taddr + it.box + c0, lo);
+        tmem_ld_wait();
+        float v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = bf16_round_f(bf16_round_f(__uint_as_float(hi[j]) + __uint_as_float(lo[j])) + b);
+        if (kUp) {
+            // even lanes hold gates, odd lanes the ups of the same channels: a lane finishes one column of each pair
+            const bool odd = lane & 1;
+#pragma unroll
+            for (int j = 0; j < 8; j += 2) {
+                const float other = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 1], 1);
+                const int c = c0 + j + int(odd);
+                if (live && c < it.rows && (row | 1) < p.rows)
+                    p.act_out[size_t(it.row0 + c) * (p.rows >> 1) + (row >> 1)] =
+                        __ushort_as_half(uint16_t(rx_swiglu_f16(odd ? other : v[j], odd ? v[j + 1] : other, p.limit)));
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                if (c0 + j >= it.rows) break;
+                const size_t at = size_t(p.sorted[it.row0 + c0 + j]) * p.rows + row;
+                if (!live) continue;
+                if (p.vals_bf16) reinterpret_cast<__nv_bfloat16*>(p.vals_out)[at] = __float2bfloat16_rn(v[j]);   // exact
+                else p.vals_out[at] = v[j];
+            }
+        }
+    }
 }
 
 template <bool kUp>
 __global__ void __launch_bounds__(kRxThreads, 1)
 moe_mxr_kernel(const RxParams p, const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap q_map,
-               const int q_rows)
+               const __grid_constant__ CUtensorMap q_map_small, const __grid_constant__ CUtensorMap q_map_mid, const int q_rows)
 {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -107,7 +164,7 @@ moe_mxr_kernel(const RxParams p, const __grid_constant__ CUtensorMap w_map, cons
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int s = 0; s < kRxStages; ++s) {
             mbar_init(&full[s], 1);
@@ -130,13 +187,13 @@ moe_mxr_kernel(const RxParams p, const __grid_constant__ CUtensorMap w_map, cons
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     const uint32_t tmem_sfx = tmem_base + 2 * kRxN, tmem_sfw = tmem_sfx + 4;
     const int items = tile_prefix[p.experts] * p.ntiles;
 
     if (warp == 0) {
         // ------------------------------------------------------------ producer
-        if (lane == 0) {
+        if (elect_one()) {
             // One thread feeds the whole pipeline, so its loop carries no divisions: the stage
             // index, its parity and the prefetch cursor advance by increments.
             uint32_t s = 0, round = 0;          // stage and how many times the ring has wrapped
@@ -148,7 +205,6 @@ moe_mxr_kernel(const RxParams p, const __grid_constant__ CUtensorMap w_map, cons
                 const RxItem pi = rx_decode(p, tile_prefix, pf_item, pf_cur);
                 pf_base = p.w + (size_t((pi.expert - p.expert_base) / p.expert_div) * p.ntiles + pi.ntile) * p.kslabs * kRxPkBytes;
             }
-            constexpr uint32_t tx = kRxPkBytes + 2 * kRxATile + 3 * kMxAtom;   // the 4-bit TMA counts packed bytes
             for (int item = blockIdx.x; item < items && !*abort_flag; item += gridDim.x) {
                 const RxItem it = rx_decode(p, tile_prefix, item, cur);
                 const int se = (it.expert - p.expert_base) / p.expert_div;
@@ -157,6 +213,9 @@ moe_mxr_kernel(const RxParams p, const __grid_constant__ CUtensorMap w_map, cons
                 const uint8_t* sfx = p.sfx + size_t(it.tile) * p.kslabs * kMxAtom;
                 int wrow = int(wblock * kRxN);
                 const int arow = it.tile * kRxRows;
+                const CUtensorMap* qm = it.box == kMxBoxSmall ? &q_map_small : it.box == kMxBoxMid ? &q_map_mid : &q_map;
+                const uint32_t piece = it.box * 128;
+                const uint32_t tx = kRxPkBytes + 2 * piece + 3 * kMxAtom;   // the 4-bit TMA counts packed bytes
                 for (int ks = 0; ks < p.kslabs; ++ks, ++issued) {
                     // ask L2 for the weight blocks a few stages ahead (also across the item boundary)
                     while (pf_base && prefetched < issued + kRxPrefetch) {
@@ -173,7 +232,7 @@ moe_mxr_kernel(const RxParams p, const __grid_constant__ CUtensorMap w_map, cons
                             }
                         }
                     }
-                    if (round > 0 && !mbar_wait_bounded(&empty[s], (round - 1) & 1)) {
+                    if (round > 0 && !mbar_wait_suspended(&empty[s], (round - 1) & 1)) {
                         atomicExch(p.fault, 41);
                         *abort_flag = 1;
                         break;
@@ -182,8 +241,8 @@ moe_mxr_kernel(const RxParams p, const __grid_constant__ CUtensorMap w_map, cons
                     uint8_t* sf_s = st + 2 * kRxATile + kRxBTile;
                     mbar_expect_tx(&full[s], tx);
                     tma_load_2d(st + 2 * kRxATile, &w_map, 0, wrow, &full[s]);
-                    tma_load_2d(st, &q_map, ks * kMxSlab, arow, &full[s]);
-                    tma_load_2d(st + kRxATile, &q_map, ks * kMxSlab, q_rows + arow, &full[s]);
+                    tma_load_2d(st, qm, ks * kMxSlab, arow, &full[s]);
+                    tma_load_2d(st + piece, qm, ks * kMxSlab, q_rows + arow, &full[s]);
                     bulk_g2s(sf_s, sfx, kMxAtom, &full[s]);
                     bulk_g2s(sf_s + kMxAtom, sfw, 2 * kMxAtom, &full[s]);
                     wrow += kRxN;
@@ -198,44 +257,57 @@ moe_mxr_kernel(const RxParams p, const __grid_constant__ CUtensorMap w_map, cons
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------- MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t s = 0, phase = 0, it_n = 0;
-            // The issuing thread shares its scheduler with two epilogue warps, so its loop is
-            // kept to a few instructions per MMA: every descriptor is the stage-0 descriptor
-            // plus a stage offset and a K-block offset in the start-address field (16-byte
-            // units), and the four instruction descriptors differ only in the scale selectors.
+            bool good = true;
+            // The issuing thread shares its scheduler with two epilogue warps, so its loop is kept to a few instructions per
+            // MMA: stage-0 descriptors plus a stage offset plus constants, and four instruction descriptors that differ only
+            // in the scale selectors.
             const uint32_t ring_addr = smem_u32(ring);
-            const uint64_t hi_d0 = umma_desc_k_sw128(ring_addr), lo_d0 = umma_desc_k_sw128(ring_addr + kRxATile),
-                           w_d0 = umma_desc_k_sw128(ring_addr + 2 * kRxATile);
-            const uint64_t sfx_d0 = umma_desc_k_plain(ring_addr + 2 * kRxATile + kRxBTile, 128);
+            const uint32_t hi_d0 = mx_desc_lo(ring_addr), lo_d0 = mx_desc_lo(ring_addr + kRxATile), w_d0 = mx_desc_lo(ring_addr + 2 * kRxATile);
+            const uint32_t sfx_d0 = mx_plain_lo(ring_addr + 2 * kRxATile + kRxBTile);
             constexpr uint32_t kStageUnits = kRxStageBytes >> 4, kAtomUnits = kMxAtom >> 4;
             // A = e4m3 pieces (rows), B = e2m1 weights
-            const uint32_t idesc0 = mx_idesc_fmt(kMxFmtE4M3, kMxFmtE2M1, kRxRows, kRxN, 0);
-            for (int item = blockIdx.x; item < items && !*abort_flag; item += gridDim.x, ++it_n) {
+            constexpr uint32_t idesc0 = mx_idesc_fmt(kMxFmtE4M3, kMxFmtE2M1, kRxRows, kRxN, 0);
+            int cur = 0;
+            for (int item = blockIdx.x; item < items && good; item += gridDim.x, ++it_n) {
+                const RxItem it = rx_decode(p, tile_prefix, item, cur);
+                const bool rows_as_m = it.box == kRxRows;
+                // small tiles: A = weights, B = both pieces of the rows
+                const uint32_t idesc_w = mx_idesc_fmt(kMxFmtE2M1, kMxFmtE4M3, kRxRows, 2 * it.box, 0);
                 const uint32_t buf = it_n & 1;
-                if (it_n >= 2 && !mbar_wait_bounded(&acc_empty[buf], ((it_n >> 1) - 1) & 1)) {
+                if (it_n >= 2 && !mbar_wait_suspended(&acc_empty[buf], ((it_n >> 1) - 1) & 1)) {
                     atomicExch(p.fault, 42);
-                    *abort_flag = 1;
+                    good = false;
                     break;
                 }
                 tc_fence_after();
                 const uint32_t d_addr = tmem_base + buf * kRxN;
                 for (int ks = 0; ks < p.kslabs; ++ks) {
-                    if (!mbar_wait_bounded(&full[s], phase)) {
+                    if (!mbar_wait_suspended(&full[s], phase)) {
                         atomicExch(p.fault, 43);
-                        *abort_flag = 1;
+                        good = false;
                         break;
                     }
-                    const uint64_t off = uint64_t(s * kStageUnits);
-                    const uint64_t hi_d = hi_d0 + off, lo_d = lo_d0 + off, w_d = w_d0 + off, sf_d = sfx_d0 + off;
+                    const uint32_t off = s * kStageUnits;
+                    const uint32_t hi_d = hi_d0 + off, lo_d = lo_d0 + off, w_d = w_d0 + off, sf_d = sfx_d0 + off;
                     tmem_cp_32x128b_warpx4(tmem_sfx, sf_d);
                     tmem_cp_32x128b_warpx4(tmem_sfw, sf_d + kAtomUnits);
                     tmem_cp_32x128b_warpx4(tmem_sfw + 4, sf_d + 2 * kAtomUnits);
+                    if (rows_as_m) {
 #pragma unroll
-                    for (uint32_t kb = 0; kb < 4; ++kb) {
-                        const uint32_t idesc = idesc0 + kb * ((1u << 4) | (1u << 29));
-                        umma_mx(d_addr, hi_d + 2 * kb, w_d + 2 * kb, idesc, tmem_sfx, tmem_sfw, ks > 0 || kb > 0);
-                        umma_mx(d_addr, lo_d + 2 * kb, w_d + 2 * kb, idesc, tmem_sfx, tmem_sfw, true);
+                        for (uint32_t kb = 0; kb < 4; ++kb) {
+                            const uint32_t idesc = idesc0 + kb * ((1u << 4) | (1u << 29));
+                            umma_mx(d_addr, hi_d + 2 * kb, w_d + 2 * kb, idesc, tmem_sfx, tmem_sfw, ks > 0 || kb > 0);
+                            umma_mx(d_addr, lo_d + 2 * kb, w_d + 2 * kb, idesc, tmem_sfx, tmem_sfw, true);
+                        }
+                    } else {
+#pragma unroll
+                        for (uint32_t kb = 0; kb < 4; ++kb) {
+                            const uint32_t idesc = idesc_w + kb * ((1u << 4) | (1u << 29));
+                            umma_mx(d_addr, w_d + 2 * kb, hi_d + 2 * kb, idesc, tmem_sfw, tmem_sfx, ks > 0 || kb > 0);
+                            umma_mx(d_addr + 2 * it.box, w_d + kRxRows * 8 + 2 * kb, hi_d + 2 * kb, idesc, tmem_sfw + 4, tmem_sfx, ks > 0 || kb > 0);
+                        }
                     }
                     umma_commit(&empty[s]);
                     if (++s == kRxStages) {
@@ -243,24 +315,25 @@ moe_mxr_kernel(const RxParams p, const __grid_constant__ CUtensorMap w_map, cons
                         phase ^= 1;
                     }
                 }
-                if (*abort_flag) break;
-                umma_commit(&acc_full[buf]);
+                if (good) umma_commit(&acc_full[buf]);
             }
+            if (!good) *abort_flag = 1;
         }
+        __syncwarp();
     } else if (warp < kRxFirstEpi) {
         // spare warp: keeps the epilogue warps' numbering aligned with the lane quarters
     } else {
         // ------------------------------------------------------------ epilogue
         // Warp w serves the 32-lane quarter w % 4 (a warp may only read its own quarter of
-        // tensor memory); the two warps of a quarter take alternate 16-column groups.
-        const int quarter = warp & 3, half = (warp - kRxFirstEpi) >> 2;
+        // tensor memory); the four warps of a quarter take the 16-column groups in turn.
+        const int quarter = warp & 3, group = (warp - kRxFirstEpi) >> 2;
         const int l = quarter * 32 + lane;   // TMEM lane = routed row of the tile
         uint32_t it_n = 0;
         int cur = 0;
         for (int item = blockIdx.x; item < items && !*abort_flag; item += gridDim.x, ++it_n) {
             const RxItem it = rx_decode(p, tile_prefix, item, cur);
             const uint32_t buf = it_n & 1;
-            if (!mbar_wait_bounded(&acc_full[buf], (it_n >> 1) & 1)) {
+            if (!mbar_wait_suspended(&acc_full[buf], (it_n >> 1) & 1)) {
                 atomicExch(p.fault, 45);
                 *abort_flag = 1;
                 break;
@@ -272,10 +345,15 @@ moe_mxr_kernel(const RxParams p, const __grid_constant__ CUtensorMap w_map, cons
             const int pos = it.row0 + min(l, it.rows - 1);
             const uint32_t taddr = tmem_base + (uint32_t(quarter * 32) << 16) + buf * kRxN;
             const int n0 = it.ntile * kRxN;
-            if (kUp) {
+            if (it.box != kRxRows) {
+                rx_small_epilogue<kUp>(p, it, bias, taddr + (group & 1) * 2 * it.box, (group & 1) * kRxRows + l, (group >> 1) * 8, lane);
+            } else if (kUp) {
                 __half* arow = p.act_out + size_t(pos) * (p.rows >> 1) + (n0 >> 1);
-                for (int c0 = half * 16; c0 < kRxN; c0 += 32) {
+                for (int c0 = group * 16; c0 < kRxN; c0 += 16 * kRxEpiGroups) {
                     if (n0 + c0 >= p.rows) break;   // warp-uniform
+                    float bs[16];                   // requested before the wait for the accumulator
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) bs[j] = n0 + c0 + j < p.rows ? __ldg(bias + n0 + c0 + j) : 0.f;
                     uint32_t r[16];
                     tmem_ld_32x16(taddr + c0, r);
                     tmem_ld_wait();
@@ -286,12 +364,10 @@ moe_mxr_kernel(const RxParams p, const __grid_constant__ CUtensorMap w_map, cons
                         const int nrow = n0 + c0 + 2 * q;
                         float gate = 0.f, up = 0.f;
                         if (nrow + 1 < p.rows) {
-                            gate = fminf(bf16_round_f(bf16_round_f(__uint_as_float(r[2 * q])) + bias[nrow]), p.limit);
-                            up = fminf(p.limit, fmaxf(-p.limit, bf16_round_f(bf16_round_f(__uint_as_float(r[2 * q + 1])) + bias[nrow + 1])));
+                            gate = bf16_round_f(bf16_round_f(__uint_as_float(r[2 * q])) + bs[2 * q]);
+                            up = bf16_round_f(bf16_round_f(__uint_as_float(r[2 * q + 1])) + bs[2 * q + 1]);
                         }
-                        const float sig = bf16_round_f(1.f / (1.f + expf(-bf16_round_f(1.702f * gate))));
-                        const float glu = bf16_round_f(gate * sig);
-                        const uint32_t hv = __half_as_ushort(__float2half_rn(bf16_round_f(glu * bf16_round_f(up + 1.f))));
+                        const uint32_t hv = rx_swiglu_f16(gate, up, p.limit);
                         if (q & 1) packed[q >> 1] |= hv << 16;
                         else packed[q >> 1] = hv;
                     }
@@ -305,8 +381,11 @@ moe_mxr_kernel(const RxParams p, const __grid_constant__ CUtensorMap w_map, cons
                 }
             } else {
                 float* vrow = p.vals_out + size_t(p.sorted[pos]) * p.rows + n0;
-                for (int c0 = half * 16; c0 < kRxN; c0 += 32) {
+                for (int c0 = group * 16; c0 < kRxN; c0 += 16 * kRxEpiGroups) {
                     if (n0 + c0 >= p.rows) break;   // warp-uniform
+                    float bs[16];                   // requested before the wait for the accumulator
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) bs[j] = n0 + c0 + j < p.rows ? __ldg(bias + n0 + c0 + j) : 0.f;
                     uint32_t r[16];
                     tmem_ld_32x16(taddr + c0, r);
                     tmem_ld_wait();
@@ -318,7 +397,7 @@ moe_mxr_kernel(const RxParams p, const __grid_constant__ CUtensorMap w_map, cons
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
                             const int d = n0 + c0 + 4 * q + j;
-                            vp[j] = d < p.rows ? bf16_round_f(bf16_round_f(__uint_as_float(r[4 * q + j])) + bias[d]) : 0.f;
+                            vp[j] = d < p.rows ? bf16_round_f(bf16_round_f(__uint_as_float(r[4 * q + j])) + bs[4 * q + j]) : 0.f;
                         }
                         if (p.vals_bf16) {   // the values are bf16-valued: the conversions below are exact
                             __nv_bfloat16* vb = reinterpret_cast<__nv_bfloat16*>(p.vals_out) + size_t(p.sorted[pos]) * p.rows + n0 + c0 + 4 * q;
@@ -461,8 +540,7 @@ int Moe::finish_mxr()
     return GARNET_B200_OK;
 }
 
-int Moe::launch_mxr_gemm(bool up, const MoeWorkspacePtrs& w, const void* q_map_ptr, int q_rows, int tiles_max,
-                         cudaStream_t stream)
+int Moe::launch_mxr_gemm(bool up, const MoeWorkspacePtrs& w, const QMapCache& q, int tiles_max, cudaStream_t stream)
 {
     const int pass = up ? 0 : 1;
     const PackGeom& geo = up ? geo_up : geo_down;
@@ -498,10 +576,11 @@ int Moe::launch_mxr_gemm(bool up, const MoeWorkspacePtrs& w, const void* q_map_p
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const CUtensorMap& qm = *static_cast<const CUtensorMap*>(q_map_ptr);
+    const CUtensorMap *qm = reinterpret_cast<const CUtensorMap*>(&q.maps[0]), *qs = reinterpret_cast<const CUtensorMap*>(&q.maps[1]),
+                      *qd = reinterpret_cast<const CUtensorMap*>(&q.maps[2]);
     const CUtensorMap& wm = *reinterpret_cast<const CUtensorMap*>(&mxr_w_map[pass]);
-    if (up) GB_CUDA(cudaLaunchKernelEx(&cfg, moe_mxr_kernel<true>, p, wm, qm, q_rows));
-    else GB_CUDA(cudaLaunchKernelEx(&cfg, moe_mxr_kernel<false>, p, wm, qm, q_rows));
+    if (up) GB_CUDA(cudaLaunchKernelEx(&cfg, moe_mxr_kernel<true>, p, wm, *qm, *qs, *qd, q.q_rows));
+    else GB_CUDA(cudaLaunchKernelEx(&cfg, moe_mxr_kernel<false>, p, wm, *qm, *qs, *qd, q.q_rows));
     return GARNET_B200_OK;
 }
 

@@ -413,6 +413,21 @@ def positions_in_expert(slots_expert):
     return pos, counts
 
 
+@pytest.mark.parametrize("h,inter", [(480, 256), (96, 64), (2880, 160)])
+@pytest.mark.parametrize("counts", [
+    (1, 8, 31, 32, 33, 55, 56, 57), (127, 128, 129, 159, 160, 161, 0, 184), (185, 16, 300, 0, 1, 256, 312, 313)])
+def test_block_scaled_row_tiles_of_every_size(h, inter, counts):
+    """Row tiles at the edges of the block-scaled kernel's orientations (at most 32, at most 56 rows, up to 128, an
+    expert's last rows behind full tiles), widths that end inside a 240-row weight tile; rows in no order."""
+    case = synth.moe_layer(4, h, inter, experts=8, topk=2, seed=11, bias_scale=0.1)
+    moe = build(case, layouts=moe_mod.LAYOUT_BLOCK)
+    rng = np.random.RandomState(5)
+    experts = rng.permutation(np.repeat(np.arange(8), counts)).astype(np.int32)
+    rows = torch.from_numpy(rng.standard_normal((experts.size, h)).astype(np.float32)).cuda().bfloat16().float()
+    pick = np.sort(rng.choice(experts.size, min(experts.size, 160), replace=False))
+    check_rows_in_two_halves(moe, case, rows, dev(experts), pick, f"counts {counts}")
+
+
 def test_gpt_oss_120b_layer_at_4096_tokens_per_slot_values_and_output():
     """The configuration the MoE throughput is quoted on: 4096 tokens, 128 experts, top-4
     (128 +- 11 rows per expert: many experts own a full 128-row tile and a nearly empty
