@@ -184,8 +184,8 @@ W4A16::~W4A16()
     if (stage_ws) cudaFree(stage_ws);
 }
 
-// Only the tile kernel (more than 16 rows) uses a workspace: the partial sums of its K slices.
-size_t W4A16::workspace_bytes(int m) const { return (m > 16 || m > max_rows_per_launch) ? tc_plan(geo, m).workspace : 0; }
+// What callers of the tile kernel (more than 16 rows) are told to bring; the kernel itself no longer needs it.
+size_t W4A16::workspace_bytes(int m) const { return (m > 16 || m > max_rows_per_launch) ? tc_workspace(geo, m) : 0; }
 
 int W4A16::run(const void* d_x, void* d_y, int m, void* ws, size_t ws_bytes, unsigned flags, cudaStream_t stream)
 {
@@ -193,14 +193,15 @@ int W4A16::run(const void* d_x, void* d_y, int m, void* ws, size_t ws_bytes, uns
     if (!d_x || !d_y) return fail(GARNET_B200_INVALID_VALUE, "w4a16_run: null x or y");
     if ((reinterpret_cast<uintptr_t>(d_x) & 15) || (reinterpret_cast<uintptr_t>(d_y) & 1))
         return fail(GARNET_B200_INVALID_VALUE, "w4a16_run: x must be 16-byte aligned");
-    // A workspace smaller than garnet_b200_w4a16_workspace asks for (or none) is allowed: the
-    // tile kernel then does not cut K into slices (slower on small matrices, same results
-    // up to the order of the fp32 sums).
+    // A workspace smaller than garnet_b200_w4a16_workspace asks for (or none) is allowed: the K slices of the tile kernel
+    // meet in distributed shared memory and nothing is written to it.
+    (void)ws;
+    (void)ws_bytes;
     const __nv_bfloat16* x = static_cast<const __nv_bfloat16*>(d_x);
     __nv_bfloat16* y = static_cast<__nv_bfloat16*>(d_y);
     // Above 16 rows the weights are worth expanding once per 128 rows for the tensor core.
     // (also when the rows do not fit one launch of the streaming kernel: a very long K)
-    if ((m > 16 || m > max_rows_per_launch)) return launch_tc(x, y, m, ws, ws_bytes, flags, stream);
+    if ((m > 16 || m > max_rows_per_launch)) return launch_tc(x, y, m, flags, stream);
     for (int m0 = 0; m0 < m; m0 += max_rows_per_launch) {
         const int rows = std::min(max_rows_per_launch, m - m0);
         const int rc = launch_stream(x + size_t(m0) * geo.cols, y + size_t(m0) * geo.rows, rows, geo.rows, flags,

@@ -1,23 +1,29 @@
 // Tensor-core (tcgen05 / TMEM) tile kernel of the int4 linear, for batches above
 // the streaming kernel's 16 rows.
 //
-// The weights are the A operand: a CTA owns kATiles x 128 weight rows (8 strips per
-// A tile) and up to 128 batch rows (the UMMA N dimension).  Per 64 columns of K:
-//   producer warp   bulk-copies the packed strip-chunks (codes + scales) and issues
-//                   the TMA load of the activation tile (128-byte swizzle);
-//   8 dequant warps expand int4 -> bf16, multiply by the group scale and store the
-//                   16-byte rows into the 128-byte-swizzled K-major A tile
-//                   (the row interleave of the packed layout makes those stores
-//                   bank-conflict free);
-//   MMA warp        one thread issues 4 x kATiles tcgen05.mma (M=128, N=batch tile,
-//                   K=16) into the TMEM accumulator and commits to the stage barrier;
-//   4 epilogue warps read the accumulator with tcgen05.ld, round to bf16 and store
-//                   y[m, n]; accumulators are double buffered so the next tile's
-//                   main loop overlaps the epilogue.
+// The weights are the A operand and live in tensor memory: a CTA owns a panel of 128 weight rows (8 strips) and a tile of up to
+// 192 batch rows (the UMMA N dimension).  Per 64 columns of K:
+//   pack producer   TMA of the packed strip-chunks (codes + scales) of 128 columns, L2 prefetch ahead of it;
+//   x producer      TMA of the activation tile (128-byte swizzle), the only operand that the MMAs read from shared memory;
+//   dequant warps   a lane owns a weight row: 64 codes -> bf16 x group scale -> tcgen05.st into one of four A tiles; four
+//                   groups of four warps, so that a warp has four steps' time for its chain, or two groups when a CTA has one
+//                   item (and half of the registers, so that two CTAs share an SM: the next launch's weights are on their way);
+//   MMA warp        one thread issues 4 tcgen05.mma (A in tensor memory, K = 16);
+//   4 epilogue      read the accumulator with tcgen05.ld, round to bf16 and store y[m, n]; accumulators are double
+//   warps           buffered so that the next tile's main loop overlaps the epilogue.
+// Small matrices are cut along K over a cluster of up to 8 CTAs, whose fp32 partial tiles meet in distributed shared memory
+// and are added in slice order: no partial sums in global memory and no second launch.
+// Bound: an MMA of N columns takes N / 2 clocks and reads N x 32 bytes; expanding through shared memory instead (the form
+// before: 32 KiB written and 48 KiB read per 128 x 256 x 64 step, a proxy fence per warp and step) took 1535 clocks per step
+// against 512 of MMAs.  Batch tiles are even shares of the batch in multiples of 16 rows, so little of them is padding.
+//   rows x K -> N             before      now (called from Python; x [1000, 2048]: 825 TFLOP/s)
+//   1000 x 2048 -> 12288      75.0 us     61.0 us
+//     77 x 2048 -> 4096       15.6 us     9.7 us
+//     16 x 6144 -> 2048       17.6 us     8.3 us
 // Numerics: w = bf16(q * s) (one rounding of the dequantised weight), products
 // exact, fp32 accumulation in TMEM, bf16 output.
 #include <algorithm>
-#include <cstdlib>
+#include <cooperative_groups.h>
 
 #include "layout.h"
 #include "tc_common.cuh"
@@ -25,69 +31,63 @@
 
 namespace gb200 {
 
-constexpr int kTcTokens = 128;            // batch rows per tile (UMMA N, multiple of 16)
-// Ring depths.  A (expanded weights) only has to cover the dequant -> MMA hand-off;
-// B (activations, from L2 through TMA) has to cover about a microsecond of L2
-// latency at ~0.4 us per 64-column tile; the packed ring is fed from L2 as well,
-// because the producer prefetches packed chunks into L2 well ahead of their use.
-__host__ __device__ constexpr int tc_a_stages(int atiles) { return atiles == 2 ? 3 : 4; }
-__host__ __device__ constexpr int tc_b_stages(int atiles) { return atiles == 2 ? 4 : 6; }
+namespace cg = cooperative_groups;
+
+constexpr int kTcMaxRows = 192;           // batch rows per tile (UMMA N): two accumulators and four A tiles fill 512 columns
+constexpr int kTcAStages = 4;             // A tiles of 64 columns of K in tensor memory, 32 columns each
+constexpr int kTcBStages = 6;             // activation tiles of 64 columns of K
+constexpr int kTcPackStages = 4;          // packed chunks of 128 columns of K
 constexpr int kTcPrefetchChunks = 8;      // packed chunks prefetched into L2 ahead of the ring
-// Packed ring depth, in 128-column chunks.  The codes come from HBM (microseconds
-// of latency against ~0.3 us per 64-column tile), so this ring is the deep one.
-__host__ __device__ constexpr int tc_pack_stages(int atiles) { return atiles == 2 ? 3 : 4; }
-// One dequant warp per strip of the CTA tile (8 per 128-row A tile): the expansion
-// of a 64-column tile is then one 16-byte unit per lane, and the 16 warps of a
-// 256-row tile keep all four schedulers busy.
-__host__ __device__ constexpr int tc_dequant_warps(int atiles) { return 8 * atiles; }
-constexpr int kTcEpilogueWarps = 4;
-constexpr int kTcFirstDequantWarp = 3;    // warp 0: packed producer, 1: MMA, 2: activation producer
-__host__ __device__ constexpr int tc_threads(int atiles)
-{
-    return (kTcFirstDequantWarp + tc_dequant_warps(atiles) + kTcEpilogueWarps) * 32;
-}
+constexpr int kTcMaxSlices = 8;           // CTAs of a cluster
+constexpr int kTcFirstDequant = 4, kTcEpilogueWarps = 4;
+__host__ __device__ constexpr int tc_threads(int groups) { return (kTcFirstDequant + 4 * groups + kTcEpilogueWarps) * 32; }
 constexpr int kTcChunkBytes = 1024 + 32;  // int4 strip-chunk
-constexpr int kTcTileBytes = 128 * 128;   // one 128-row x 64-column 16-bit tile
+constexpr int kTcPackBytes = 8 * kTcChunkBytes;
+constexpr uint32_t kTcACols = 32;
+// Tensor memory: two accumulators and the A tiles, or, when a CTA has one item of at most 128 rows, one accumulator and the A
+// tiles in half of it, so that the next launch's CTA can move in (its weights are on their way while this one finishes).
+constexpr int kTcHalfRows = 128;
+static_assert(2 * kTcMaxRows + kTcAStages * kTcACols <= 512 && kTcHalfRows + kTcAStages * kTcACols <= 256, "tensor memory");
 
 struct TcParams {
     const uint8_t* packed;
     __nv_bfloat16* y;
     int* fault;
-    int m, n, k;
+    int m, n;
     int ldy;
-    int strips_padded, chunks;
-    int panels, token_tiles;
-    int kslices, chunks_per_slice;   // the K dimension of a tile may be cut into slices handled by different CTAs
-    float* partial;                  // [kslices][m][n] fp32 partial sums (kslices > 1), else nullptr
+    int chunks;
+    int panels, row_tiles, tile_rows;
+    int kslices, chunks_per_slice;   // the K dimension of a tile may be cut into slices handled by the CTAs of a cluster
     int scale_dtype;
+    int tmem_cols, col_a;            // tensor memory: columns, and where the A tiles start
 };
 
 // Work item -> (panel, batch tile, K slice) and the slice's chunk range.
 struct TcItem {
     int panel, tt, c0, c1;
-    int slice;
 };
 __device__ __forceinline__ TcItem tc_decode(const TcParams& p, int item)
 {
     TcItem it;
-    const int per_panel = p.token_tiles * p.kslices;
+    const int per_panel = p.row_tiles * p.kslices;
     it.panel = item / per_panel;
     const int rem = item - it.panel * per_panel;
     it.tt = rem / p.kslices;
-    it.slice = rem - it.tt * p.kslices;
-    it.c0 = it.slice * p.chunks_per_slice;
+    const int slice = rem - it.tt * p.kslices;
+    it.c0 = slice * p.chunks_per_slice;
     it.c1 = min(p.chunks, it.c0 + p.chunks_per_slice);
     return it;
 }
 
-template <int kATiles>
+// Shared memory: packed ring, barriers, activation ring (a stage is tile_rows x 128 bytes).  The partial tile of a K slice,
+// [batch row][128 weight rows] fp32, takes the activation ring's place.
 struct TcSmem {
-    static constexpr int a = 0;
-    static constexpr int b = a + tc_a_stages(kATiles) * kATiles * kTcTileBytes;
-    static constexpr int pk = b + tc_b_stages(kATiles) * kTcTileBytes;
-    static constexpr int bars = pk + tc_pack_stages(kATiles) * kATiles * 8 * kTcChunkBytes;
-    static constexpr int total = bars + 256 + 1024;   // barriers + slack for 1024-byte alignment
+    static constexpr int pk = 0;
+    static constexpr int bars = pk + kTcPackStages * kTcPackBytes;
+    static constexpr int b = (bars + 256 + 1023) / 1024 * 1024;
+    static constexpr int total(int tile_rows) { return b + kTcBStages * tile_rows * 128 + 1024; }   // slack for 1024-byte alignment
 };
+static_assert(128 * 4 <= kTcBStages * 128, "partial tile");
 
 // One int4 word (8 codes of one row, pair-interleaved) times a scale -> 8 bf16.
 __device__ __forceinline__ uint4 int4_word_to_bf16x8(uint32_t w, uint32_t scale_bf16x2)
@@ -115,48 +115,87 @@ __device__ __forceinline__ uint4 int4_word_to_bf16x8_f32(uint32_t w, float s)
     return make_uint4(out[0], out[1], out[2], out[3]);
 }
 
-template <int kATiles>
-__global__ void __launch_bounds__(tc_threads(kATiles), 1)
-w4a16_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap x_map,
-                const __grid_constant__ CUtensorMap w_map)
+// D[tmem] (+)= A[tmem] * B[smem]; the descriptor comes as its low word (tc_desc_lo), so that the issuing thread adds one
+// constant per MMA.
+constexpr uint32_t kTcDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t tc_desc_lo(uint32_t smem_addr) { return ((smem_addr & 0x3FFFFu) >> 4) | (1u << 16); }
+__device__ __forceinline__ void tc_umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc, bool accumulate)
 {
-    using S = TcSmem<kATiles>;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\t"
+        "mov.b64 b, {%2, %5};\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n\t}" ::"r"(d_tmem),
+        "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(uint32_t(accumulate)), "n"(kTcDescHi)
+        : "memory");
+}
+__device__ __forceinline__ void tc_st_32x32(uint32_t taddr, const uint4 (&v)[8])
+{
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
+        "r"(v[0].x), "r"(v[0].y), "r"(v[0].z), "r"(v[0].w), "r"(v[1].x), "r"(v[1].y), "r"(v[1].z), "r"(v[1].w), "r"(v[2].x), "r"(v[2].y),
+        "r"(v[2].z), "r"(v[2].w), "r"(v[3].x), "r"(v[3].y), "r"(v[3].z), "r"(v[3].w), "r"(v[4].x), "r"(v[4].y), "r"(v[4].z), "r"(v[4].w),
+        "r"(v[5].x), "r"(v[5].y), "r"(v[5].z), "r"(v[5].w), "r"(v[6].x), "r"(v[6].y), "r"(v[6].z), "r"(v[6].w), "r"(v[7].x), "r"(v[7].y),
+        "r"(v[7].z), "r"(v[7].w)
+        : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tc_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+    tmem_ld_wait();
+}
+// y[row, n], y[row, n + 1] of a pair of neighbouring outputs.
+__device__ __forceinline__ void tc_store_pair(const TcParams& p, int row, int n, float a, float b, bool wide)
+{
+    __nv_bfloat16* at = p.y + size_t(row) * p.ldy + n;
+    const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+    if (wide && n + 1 < p.n) *reinterpret_cast<__nv_bfloat162*>(at) = v;
+    else {
+        if (n < p.n) at[0] = v.x;
+        if (n + 1 < p.n) at[1] = v.y;
+    }
+}
+
+template <int kGroups>
+__global__ void __launch_bounds__(tc_threads(kGroups), 4 / kGroups)
+w4a16_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map)
+{
+    constexpr int kTcThreads = tc_threads(kGroups), kTcFirstEpilogue = kTcFirstDequant + 4 * kGroups;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t* a_ring = smem + S::a;
-    uint8_t* b_ring = smem + S::b;
-    uint8_t* pk_ring = smem + S::pk;
-    constexpr int kTcPackStages = tc_pack_stages(kATiles);
-    constexpr int kAStages = tc_a_stages(kATiles);
-    constexpr int kBStages = tc_b_stages(kATiles);
-    constexpr int kTcDequantWarps = tc_dequant_warps(kATiles);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::bars);
+    uint8_t* b_ring = smem + TcSmem::b;
+    uint8_t* pk_ring = smem + TcSmem::pk;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + TcSmem::bars);
     uint64_t* pk_full = bars;                          // [kTcPackStages]
     uint64_t* pk_empty = pk_full + kTcPackStages;      // [kTcPackStages]
-    uint64_t* a_full = pk_empty + kTcPackStages;       // [kAStages]
-    uint64_t* a_empty = a_full + kAStages;             // [kAStages]
-    uint64_t* b_full = a_empty + kAStages;             // [kBStages]
-    uint64_t* b_empty = b_full + kBStages;             // [kBStages]
-    uint64_t* acc_full = b_empty + kBStages;           // [2]
+    uint64_t* a_full = pk_empty + kTcPackStages;       // [kTcAStages]
+    uint64_t* a_empty = a_full + kTcAStages;           // [kTcAStages]
+    uint64_t* b_full = a_empty + kTcAStages;           // [kTcBStages]
+    uint64_t* b_empty = b_full + kTcBStages;           // [kTcBStages]
+    uint64_t* acc_full = b_empty + kTcBStages;         // [2]
     uint64_t* acc_empty = acc_full + 2;                // [2]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    constexpr int kStripsPerPanel = 8 * kATiles;
-    constexpr int kPackStageBytes = kStripsPerPanel * kTcChunkBytes;
-    constexpr uint32_t kTmemCols = 2 * kATiles * 128;   // two accumulator buffers
-
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int s = 0; s < kTcPackStages; ++s) {
             mbar_init(&pk_full[s], 1);
-            mbar_init(&pk_empty[s], kTcDequantWarps);
+            mbar_init(&pk_empty[s], 8);   // four warps per half of the chunk
         }
-        for (int s = 0; s < kAStages; ++s) {
-            mbar_init(&a_full[s], kTcDequantWarps);
+        for (int s = 0; s < kTcAStages; ++s) {
+            mbar_init(&a_full[s], 4);
             mbar_init(&a_empty[s], 1);
         }
-        for (int s = 0; s < kBStages; ++s) {
+        for (int s = 0; s < kTcBStages; ++s) {
             mbar_init(&b_full[s], 1);
             mbar_init(&b_empty[s], 1);
         }
@@ -168,22 +207,22 @@ w4a16_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap x_map,
         fence_barrier_init();
     }
     if (warp == 1) {
-        tmem_alloc(tmem_slot, kTmemCols);
+        tmem_alloc(tmem_slot, p.tmem_cols);
         tmem_relinquish();
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     pdl_launch_dependents();
 
-    const int items = p.panels * p.token_tiles * p.kslices;
+    const int items = p.panels * p.row_tiles * p.kslices;
 
     if (warp == 0) {
         // ------------------------------------- producer of packed codes + scales
         // Weights are constants: this stream starts before the previous kernel in the
         // stream has finished, and runs as far ahead as its ring allows.
-        if (lane == 0) {
+        if (elect_one()) {
             // One thread feeds the ring, so its loop carries no divisions: the stage index, the
             // ring's wrap count and the prefetch cursor advance by increments.
             uint32_t ps = 0, round = 0, issued = 0, prefetched = 0;
@@ -192,11 +231,10 @@ w4a16_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap x_map,
             int pf_c = pf.c0;
             for (int item = blockIdx.x; item < items && !*abort_flag; item += gridDim.x) {
                 const TcItem it = tc_decode(p, item);
-                const int strip0 = it.panel * kStripsPerPanel;
                 for (int c = it.c0; c < it.c1; ++c, ++issued) {
                     // keep the L2 prefetch kTcPrefetchChunks ahead of the ring, across items
                     while (pf_item < items && prefetched < issued + kTcPrefetchChunks) {
-                        tma_prefetch_2d(&w_map, pf_c * (kTcChunkBytes / 8), pf.panel * kStripsPerPanel);
+                        tma_prefetch_2d(&w_map, pf_c * (kTcChunkBytes / 8), pf.panel * 8);
                         ++prefetched;
                         if (++pf_c == pf.c1) {
                             pf_item += gridDim.x;
@@ -206,15 +244,14 @@ w4a16_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap x_map,
                             }
                         }
                     }
-                    if (round > 0 && !mbar_wait_bounded(&pk_empty[ps], (round - 1) & 1)) {
+                    if (round > 0 && !mbar_wait_suspended(&pk_empty[ps], (round - 1) & 1)) {
                         atomicExch(p.fault, 11);
                         *abort_flag = 1;
                         break;
                     }
-                    // one TMA operation fetches chunk c of all the panel's strips (rows
-                    // past the last strip are filled with zeros and count as bytes)
-                    mbar_expect_tx(&pk_full[ps], kPackStageBytes);
-                    tma_load_2d(pk_ring + ps * kPackStageBytes, &w_map, c * (kTcChunkBytes / 8), strip0, &pk_full[ps]);
+                    // one TMA operation fetches chunk c of all the panel's strips
+                    mbar_expect_tx(&pk_full[ps], kTcPackBytes);
+                    tma_load_2d(pk_ring + ps * kTcPackBytes, &w_map, c * (kTcChunkBytes / 8), it.panel * 8, &pk_full[ps]);
                     if (++ps == kTcPackStages) {
                         ps = 0;
                         ++round;
@@ -224,195 +261,151 @@ w4a16_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap x_map,
         }
     } else if (warp == 2) {
         // ------------------------------------------ producer of activation tiles
-        if (lane == 0) {
-            uint32_t ab_n = 0;
+        if (elect_one()) {
+            uint32_t s = 0, round = 0;
+            const uint32_t bytes = p.tile_rows * 128;
             pdl_wait();   // activations come from the previous kernel in the stream
             for (int item = blockIdx.x; item < items && !*abort_flag; item += gridDim.x) {
                 const TcItem it = tc_decode(p, item);
-                const int tt = it.tt;
                 for (int kt = 2 * it.c0; kt < 2 * it.c1; ++kt) {
-                    const uint32_t s = ab_n % kBStages;
-                    if (ab_n >= kBStages && !mbar_wait_bounded(&b_empty[s], ((ab_n / kBStages) - 1) & 1)) {
+                    if (round > 0 && !mbar_wait_suspended(&b_empty[s], (round - 1) & 1)) {
                         atomicExch(p.fault, 12);
                         *abort_flag = 1;
                         break;
                     }
-                    mbar_expect_tx(&b_full[s], kTcTileBytes);
-                    tma_load_2d(b_ring + s * kTcTileBytes, &x_map, kt * 64, tt * kTcTokens, &b_full[s]);
-                    ++ab_n;
+                    mbar_expect_tx(&b_full[s], bytes);
+                    tma_load_2d(b_ring + s * bytes, &x_map, kt * 64, it.tt * p.tile_rows, &b_full[s]);
+                    if (++s == kTcBStages) s = 0, ++round;
                 }
             }
         }
     } else if (warp == 1) {
         // ----------------------------------------------------------- MMA issuer
-        if (lane == 0) {
-            uint32_t ab_n = 0, it_n = 0;
-            for (int item = blockIdx.x; item < items && !*abort_flag; item += gridDim.x, ++it_n) {
-                                // UMMA M = 128 batch rows (TMEM lanes), N = the tile's weight rows (TMEM columns)
-                const uint32_t idesc = umma_idesc_f16(1, kTcTokens, kATiles * 128);
+        if (elect_one()) {
+            uint32_t s = 0, a_phase = 0, sb = 0, b_phase = 0, it_n = 0;
+            bool good = true;
+            // UMMA M = 128 weight rows (TMEM lanes), N = the tile's batch rows (TMEM columns)
+            const uint32_t idesc = umma_idesc_f16(1, 128, p.tile_rows);
+            const uint32_t b0 = tc_desc_lo(smem_u32(b_ring));
+            for (int item = blockIdx.x; item < items && good; item += gridDim.x, ++it_n) {
                 const uint32_t buf = it_n & 1;
-                if (it_n >= 2 && !mbar_wait_bounded(&acc_empty[buf], ((it_n >> 1) - 1) & 1)) {
+                if (it_n >= 2 && !mbar_wait_suspended(&acc_empty[buf], ((it_n >> 1) - 1) & 1)) {
                     atomicExch(p.fault, 13);
-                    *abort_flag = 1;
+                    good = false;
                     break;
                 }
                 tc_fence_after();
                 const TcItem it = tc_decode(p, item);
                 const int ktiles = 2 * (it.c1 - it.c0);
+                const uint32_t d = tmem_base + buf * kTcMaxRows;
                 for (int kt = 0; kt < ktiles; ++kt) {
-                    const uint32_t s = ab_n % kAStages, sb = ab_n % kBStages;
-                    if (!mbar_wait_bounded(&a_full[s], (ab_n / kAStages) & 1) ||
-                        !mbar_wait_bounded(&b_full[sb], (ab_n / kBStages) & 1)) {
+                    if (!mbar_wait_suspended(&b_full[sb], b_phase) || !mbar_wait_suspended(&a_full[s], a_phase)) {
                         atomicExch(p.fault, 14);
-                        *abort_flag = 1;
+                        good = false;
                         break;
                     }
                     tc_fence_after();
-                    // The activation tile is the UMMA A operand; the expanded weight tiles of
-                    // the stage are contiguous and form one B operand of kATiles*128 rows.  One
-                    // instruction per 16 columns of K reads 4 KiB + kATiles*4 KiB of shared memory.
-                    const uint32_t x_addr = smem_u32(b_ring + sb * kTcTileBytes);
-                    const uint32_t w_addr = smem_u32(a_ring + s * kATiles * kTcTileBytes);
+                    const uint32_t a = tmem_base + p.col_a + s * kTcACols, b = b0 + sb * (p.tile_rows * 128 >> 4);
 #pragma unroll
-                    for (int k16 = 0; k16 < 4; ++k16)
-                        umma_f16(tmem_base + buf * (kATiles * 128), umma_desc_k_sw128(x_addr + k16 * 32),
-                                 umma_desc_k_sw128(w_addr + k16 * 32), idesc, kt > 0 || k16 > 0);
+                    for (int k16 = 0; k16 < 4; ++k16) tc_umma_ts(d, a + k16 * 8, b + k16 * 2, idesc, kt > 0 || k16 > 0);
                     umma_commit(&a_empty[s]);    // stages reusable once these MMAs have read them
                     umma_commit(&b_empty[sb]);
-                    ++ab_n;
+                    if (++s == kTcAStages) s = 0, a_phase ^= 1;
+                    if (++sb == kTcBStages) sb = 0, b_phase ^= 1;
                 }
-                if (*abort_flag) break;
-                umma_commit(&acc_full[buf]);
+                if (good) umma_commit(&acc_full[buf]);
             }
+            if (!good) *abort_flag = 1;
         }
-    } else if (warp < kTcFirstDequantWarp + kTcDequantWarps) {
+    } else if (warp >= kTcFirstDequant && warp < kTcFirstEpilogue) {
         // -------------------------------------------------------------- dequant
-        const int dq = warp - kTcFirstDequantWarp;
-        const int g = lane >> 2, t = lane & 3;
-        uint32_t pk_n = 0, ab_n = 0;
+        // A group of four warps expands every kGroups-th 64 columns (half of every chunk or of every other chunk) into A tile
+        // 2 (chunk % 2) + half.  Warp w writes the 32-lane quarter w % 4 (the only one it may), lane = weight row: two strips of
+        // 16 rows per warp.  Rows r and r + 8 of a strip share their 16-byte units (words x, z and y, w), which their two lanes
+        // read together.
+        const int quarter = warp & 3, group = (warp - kTcFirstDequant) >> 2, half = group & 1;
+        const int strip = 2 * quarter + (lane >> 4), r = lane & 15, g = ((r & 3) << 1) | ((r >> 2) & 1);   // row_of_g(g) == r & 7
+        const bool upper = r >= 8;
+        const uint8_t* units = pk_ring + strip * kTcChunkBytes + half * 512 + g * 64;
+        const uint8_t* scales = pk_ring + strip * kTcChunkBytes + 1024 + g * 4 + (upper ? 2 : 0);
+        const uint32_t a_tiles = tmem_base + (uint32_t(quarter * 32) << 16) + p.col_a;
+        uint32_t n = 0;   // chunks that have gone by
         for (int item = blockIdx.x; item < items && !*abort_flag; item += gridDim.x) {
             const TcItem it = tc_decode(p, item);
-            const int panel = it.panel;
-            const int valid = min(kStripsPerPanel, p.strips_padded - panel * kStripsPerPanel);
-            for (int c = it.c0; c < it.c1 && !*abort_flag; ++c) {
-                const uint32_t ps = pk_n % kTcPackStages;
-                if (!mbar_wait_bounded(&pk_full[ps], (pk_n / kTcPackStages) & 1)) {
+            for (int c = it.c0; c < it.c1; ++c, ++n) {
+                if (kGroups == 4 && int(n & 1) != group >> 1) continue;
+                const uint32_t tile = 2 * (n & 1) + half;
+                const uint32_t ps = n % kTcPackStages;
+                if (!mbar_wait_suspended(&pk_full[ps], (n / kTcPackStages) & 1)) {
                     atomicExch(p.fault, 15);
                     *abort_flag = 1;
                     break;
                 }
-                const uint8_t* pk = pk_ring + ps * kPackStageBytes;
+                uint32_t w[8];
 #pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    const uint32_t s = ab_n % kAStages;
-                    if (ab_n >= kAStages && !mbar_wait_bounded(&a_empty[s], ((ab_n / kAStages) - 1) & 1)) {
-                        atomicExch(p.fault, 16);
-                        *abort_flag = 1;
-                        break;
-                    }
-                    tc_fence_after();
-                    {
-                        const int sidx = dq, at = dq >> 3;   // this warp's strip, and the A tile it belongs to
-                        if (sidx < valid) {
-                            const uint8_t* sc = pk + sidx * kTcChunkBytes;
-                            const uint4 u = *reinterpret_cast<const uint4*>(sc + half * 512 + lane * 16);
-                            const uint32_t sw = *reinterpret_cast<const uint32_t*>(sc + 1024 + g * 4);
-                            uint4 v0, v1, v2, v3;
-                            if (p.scale_dtype == GARNET_B200_BF16) {
-                                const uint32_t s_lo = (sw & 0xffffu) * 0x10001u, s_hi = (sw >> 16) * 0x10001u;
-                                v0 = int4_word_to_bf16x8(u.x, s_lo);
-                                v1 = int4_word_to_bf16x8(u.y, s_hi);
-                                v2 = int4_word_to_bf16x8(u.z, s_lo);
-                                v3 = int4_word_to_bf16x8(u.w, s_hi);
-                            } else {
-                                const float f_lo = __half2float(__ushort_as_half(uint16_t(sw & 0xffffu)));
-                                const float f_hi = __half2float(__ushort_as_half(uint16_t(sw >> 16)));
-                                v0 = int4_word_to_bf16x8_f32(u.x, f_lo);
-                                v1 = int4_word_to_bf16x8_f32(u.y, f_hi);
-                                v2 = int4_word_to_bf16x8_f32(u.z, f_lo);
-                                v3 = int4_word_to_bf16x8_f32(u.w, f_hi);
-                            }
-                            // rows R(g), R(g)+8 of strip dq; 16-byte chunks t and t+4, XOR-swizzled by row % 8
-                            uint8_t* tile = a_ring + (s * kATiles + at) * kTcTileBytes;
-                            const int r0 = (dq & 7) * 16 + row_of_g(g), r1 = r0 + 8;
-                            const int x0 = r0 & 7;   // == r1 & 7
-                            *reinterpret_cast<uint4*>(tile + r0 * 128 + ((t ^ x0) << 4)) = v0;
-                            *reinterpret_cast<uint4*>(tile + r1 * 128 + ((t ^ x0) << 4)) = v1;
-                            *reinterpret_cast<uint4*>(tile + r0 * 128 + (((t + 4) ^ x0) << 4)) = v2;
-                            *reinterpret_cast<uint4*>(tile + r1 * 128 + (((t + 4) ^ x0) << 4)) = v3;
-                        }
-                    }
-                    fence_proxy_async_smem();   // generic-proxy stores -> visible to the tensor core
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&a_full[s]);
-                    ++ab_n;
+                for (int t = 0; t < 4; ++t) {
+                    const uint4 u = *reinterpret_cast<const uint4*>(units + ps * kTcPackBytes + t * 16);
+                    w[t] = upper ? u.y : u.x;
+                    w[4 + t] = upper ? u.w : u.z;
                 }
+                const uint32_t sw = *reinterpret_cast<const uint16_t*>(scales + ps * kTcPackBytes);
+                uint4 v[8];
+                if (p.scale_dtype == GARNET_B200_BF16) {
+#pragma unroll
+                    for (int t = 0; t < 8; ++t) v[t] = int4_word_to_bf16x8(w[t], sw * 0x10001u);
+                } else {
+                    const float f = __half2float(__ushort_as_half(uint16_t(sw)));
+#pragma unroll
+                    for (int t = 0; t < 8; ++t) v[t] = int4_word_to_bf16x8_f32(w[t], f);
+                }
+                if (n >= 2 && !mbar_wait_suspended(&a_empty[tile], ((n >> 1) - 1) & 1)) {
+                    atomicExch(p.fault, 16);
+                    *abort_flag = 1;
+                    break;
+                }
+                tc_fence_after();
+                tc_st_32x32(a_tiles + tile * kTcACols, v);
+                tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&pk_empty[ps]);
-                ++pk_n;
+                // The packed stage is given back only here, where the loaded values have been used: right after the loads the
+                // arrival can overtake them in the shared-memory queue, and the next TMA then overwrites what they read.
+                if (lane == 0) mbar_arrive(&pk_empty[ps]), mbar_arrive(&a_full[tile]);
             }
         }
-    } else {
+    } else if (warp >= kTcFirstEpilogue) {
         // ------------------------------------------------------------- epilogue
         const int quarter = warp & 3;   // TMEM lanes 32*quarter .. +31 belong to this warp
+        const bool wide = (p.ldy & 1) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 3) == 0, odd = lane & 1;
         uint32_t it_n = 0;
-        bool waited = false;
         for (int item = blockIdx.x; item < items && !*abort_flag; item += gridDim.x, ++it_n) {
             const TcItem it = tc_decode(p, item);
-            const int panel = it.panel, tt = it.tt;
             const uint32_t buf = it_n & 1;
-            if (!mbar_wait_bounded(&acc_full[buf], (it_n >> 1) & 1)) {
+            if (!mbar_wait_suspended(&acc_full[buf], (it_n >> 1) & 1)) {
                 atomicExch(p.fault, 17);
                 *abort_flag = 1;
                 break;
             }
             tc_fence_after();
-            if (!waited) {
-                pdl_wait();   // y may still be read by the previous kernel in the stream
-                waited = true;
-            }
-            // TMEM lane = batch row of the tile, column = weight row of the panel: a thread
-            // reads 32 consecutive outputs of its row and stores them as 64 contiguous bytes.
-            const int m = tt * kTcTokens + quarter * 32 + lane;
-            __nv_bfloat16* yrow = p.y + size_t(min(m, p.m - 1)) * p.ldy;
-            const bool vec_ok = (p.ldy & 7) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 15) == 0;
-            for (int c0 = 0; c0 < kATiles * 128; c0 += 32) {
-                const int n0 = panel * (kATiles * 128) + c0;
-                if (n0 >= p.n) break;   // warp-uniform
-                uint32_t r[32];
-                tmem_ld_32x32(tmem_base + (uint32_t(quarter * 32) << 16) + buf * (kATiles * 128) + c0, r);
-                tmem_ld_wait();
-                if (m >= p.m) continue;
-                if (p.partial) {
-                    // a K slice: fp32 partial sums, added up in slice order by the reduction kernel
-                    float* prow = p.partial + (size_t(it.slice) * p.m + m) * p.n;
-                    if (n0 + 32 <= p.n && (p.n & 3) == 0) {
+            if (it_n == 0) pdl_wait();   // y may still be read by the previous kernel in the stream
+            // TMEM lane = weight row of the panel, column = batch row of the tile
+            const int row0 = it.tt * p.tile_rows, rows = min(p.tile_rows, p.m - row0), n = it.panel * 128 + quarter * 32 + lane;
+            const uint32_t taddr = tmem_base + (uint32_t(quarter * 32) << 16) + buf * kTcMaxRows;
+            for (int c0 = 0; c0 < rows; c0 += 16) {
+                uint32_t v[16];
+                tc_ld_32x16(taddr + c0, v);
+                if (p.kslices > 1) {
+                    float* part = reinterpret_cast<float*>(b_ring) + size_t(c0) * 128 + quarter * 32 + lane;
 #pragma unroll
-                        for (int q = 0; q < 8; ++q)
-                            *reinterpret_cast<uint4*>(prow + n0 + 4 * q) = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            if (n0 + j < p.n) prow[n0 + j] = __uint_as_float(r[j]);
-                    }
+                    for (int j = 0; j < 16; ++j) part[j * 128] = __uint_as_float(v[j]);
                     continue;
                 }
-                if (vec_ok && n0 + 32 <= p.n) {
+                // neighbouring lanes hold neighbouring outputs of a row: each finishes one row of a pair of rows
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        uint32_t w[4];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const __nv_bfloat162 v = __floats2bfloat162_rn(__uint_as_float(r[8 * q + 2 * j]),
-                                                                           __uint_as_float(r[8 * q + 2 * j + 1]));
-                            w[j] = *reinterpret_cast<const uint32_t*>(&v);
-                        }
-                        *reinterpret_cast<uint4*>(yrow + n0 + 8 * q) = make_uint4(w[0], w[1], w[2], w[3]);
-                    }
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j)
-                        if (n0 + j < p.n) yrow[n0 + j] = __float2bfloat16_rn(__uint_as_float(r[j]));
+                for (int j = 0; j < 16; j += 2) {
+                    const float other = __uint_as_float(__shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 1], 1));
+                    const float mine = __uint_as_float(odd ? v[j + 1] : v[j]);
+                    const int c = c0 + j + int(odd);
+                    if (c < rows) tc_store_pair(p, row0 + c, n & ~1, odd ? other : mine, odd ? mine : other, wide);
                 }
             }
             tc_fence_before();
@@ -420,69 +413,79 @@ w4a16_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap x_map,
             if (lane == 0) mbar_arrive(&acc_empty[buf]);
         }
     }
+    __syncwarp();
+    if (p.kslices > 1) {
+        // One item per CTA; the cluster's CTAs hold the K slices of one tile.  The batch rows go round the CTAs, each of which
+        // adds the slices of its rows in slice order.
+        cg::cluster_group cluster = cg::this_cluster();
+        cluster.sync();
+        const TcItem it = tc_decode(p, blockIdx.x);
+        const int row0 = it.tt * p.tile_rows, rows = min(p.tile_rows, p.m - row0), rank = int(cluster.block_rank());
+        const bool wide = (p.ldy & 1) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 3) == 0;
+        const int pair = (threadIdx.x & 63) * 2;
+        if (!*abort_flag) {
+            pdl_wait();
+            for (int c = rank + int(threadIdx.x >> 6) * p.kslices; c < rows; c += (kTcThreads / 64) * p.kslices) {
+                float2 part[kTcMaxSlices], sum = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int s = 0; s < kTcMaxSlices; ++s)
+                    part[s] = s < p.kslices ? *reinterpret_cast<const float2*>(cluster.map_shared_rank(reinterpret_cast<float*>(b_ring), s) + size_t(c) * 128 + pair)
+                                            : make_float2(0.f, 0.f);
+#pragma unroll
+                for (int s = 0; s < kTcMaxSlices; ++s)
+                    if (s < p.kslices) sum.x += part[s].x, sum.y += part[s].y;
+                tc_store_pair(p, row0 + c, it.panel * 128 + pair, sum.x, sum.y, wide);
+            }
+        }
+        cluster.sync();   // peers may still read this CTA's partial tile
+    }
 
     // ---- teardown: every role arrives here, also after a wait that gave up
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, kTmemCols);
-    }
-}
-
-// y[m, n] = bf16(sum of the K slices' partial sums, in slice order).  Four outputs per thread.
-__global__ void w4a16_splitk_reduce_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ y, int m, int n, int ldy,
-                                           int slices)
-{
-    pdl_wait();   // the partial sums come from the kernel before this one
-    const size_t total = size_t(m) * n;
-    const size_t idx = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
-    if (idx >= total) return;
-    if ((n & 3) == 0 && (ldy & 3) == 0 && (reinterpret_cast<uintptr_t>(y) & 7) == 0) {
-        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int s = 0; s < slices; ++s) {
-            const float4 v = __ldcg(reinterpret_cast<const float4*>(partial + size_t(s) * total + idx));
-            sum.x += v.x;
-            sum.y += v.y;
-            sum.z += v.z;
-            sum.w += v.w;
-        }
-        const __nv_bfloat162 a = __floats2bfloat162_rn(sum.x, sum.y), b = __floats2bfloat162_rn(sum.z, sum.w);
-        *reinterpret_cast<uint2*>(y + (idx / n) * ldy + idx % n) =
-            make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
-    } else {
-        for (size_t j = idx; j < min(idx + 4, total); ++j) {
-            float sum = 0.f;
-            for (int s = 0; s < slices; ++s) sum += partial[size_t(s) * total + j];
-            y[(j / n) * ldy + j % n] = __float2bfloat16_rn(sum);
-        }
+        tmem_dealloc(tmem_base, p.tmem_cols);
     }
 }
 
 // ------------------------------------------------------------------ host side
 
-// How the tile kernel cuts the work for a batch of m rows: 256-row panels when they
-// already fill the machine, else 128-row panels, and K slices until there are about
-// as many work items as SMs.
+// How the tile kernel cuts the work for a batch of m rows: as few even shares of the batch as tiles allow or, when that is
+// more than a wave, up to three more, whichever makes the least work of whole waves (an MMA costs its N columns and some fixed
+// time, about 24 columns' worth); K slices while the machine has room for twice the CTAs.
 TcPlan tc_plan(const PackGeom& geo, int m)
 {
     TcPlan t;
-    t.token_tiles = (m + kTcTokens - 1) / kTcTokens;
-    const int panels256 = (geo.strips_padded + 15) / 16;
-    t.atiles = panels256 * t.token_tiles >= 2 * kSmCount ? 2 : 1;
-    t.panels = t.atiles == 2 ? panels256 : geo.strips_padded / 8;
-    const int tiles = t.panels * t.token_tiles;
+    t.panels = geo.strips_padded / 8;
+    const int fewest = (m + kTcMaxRows - 1) / kTcMaxRows;
+    long long best = 0;
+    for (int tiles = fewest; tiles == fewest || (tiles < fewest + 4 && t.panels * fewest > kSmCount); ++tiles) {
+        const int rows = ((m + tiles - 1) / tiles + 15) / 16 * 16;
+        const long long used = (m + rows - 1) / rows, waves = (t.panels * used + kSmCount - 1) / kSmCount, cost = waves * (rows + 24);
+        if (tiles == fewest || cost < best) best = cost, t.row_tiles = int(used), t.tile_rows = rows;
+    }
+    const long long tiles = (long long)t.panels * t.row_tiles;
+    int slices = 1;
+    while (slices < kTcMaxSlices && 2 * slices <= geo.chunks && tiles * slices * 2 <= kSmCount) slices *= 2;
+    t.chunks_per_slice = (geo.chunks + slices - 1) / slices;
+    t.kslices = (geo.chunks + t.chunks_per_slice - 1) / t.chunks_per_slice;
+    if (t.kslices != slices) t.kslices = 1, t.chunks_per_slice = geo.chunks;   // a slice would be empty
+    return t;
+}
+
+// Workspace that a call of m rows is told to bring: fp32 partial sums of the K slices, which now meet on the chip.  The size
+// stays what callers were told before.
+size_t tc_workspace(const PackGeom& geo, int m)
+{
+    const int row_tiles = (m + 127) / 128, panels256 = (geo.strips_padded + 15) / 16;
+    const int tiles = (panels256 * row_tiles >= 2 * kSmCount ? panels256 : geo.strips_padded / 8) * row_tiles;
     int want = tiles >= kSmCount ? 1 : (kSmCount + tiles - 1) / tiles;
     want = std::min(want, std::min(geo.chunks, 16));
-    // every slice writes and the last one re-reads m x n fp32 partial sums: beyond a few MB per
-    // slice that costs more than the idle SMs it saves
     const size_t plane = size_t(m) * geo.rows * sizeof(float);
     want = int(std::max<size_t>(1, std::min<size_t>(size_t(want), (size_t(6) << 20) / std::max<size_t>(plane, 1))));
-
-    t.chunks_per_slice = (geo.chunks + want - 1) / want;
-    t.kslices = (geo.chunks + t.chunks_per_slice - 1) / t.chunks_per_slice;
-    t.workspace = t.kslices > 1 ? size_t(t.kslices) * m * geo.rows * sizeof(float) : 0;
-    return t;
+    const int per_slice = (geo.chunks + want - 1) / want, slices = (geo.chunks + per_slice - 1) / per_slice;
+    return slices > 1 ? slices * plane : 0;
 }
 
 TensorMapEncodeFn tensor_map_encoder()
@@ -531,65 +534,58 @@ int make_tensor_map_2d_bytes(CUtensorMap* map, const void* base, uint64_t rows, 
 
 int W4A16::init_tc()
 {
-    static_assert(sizeof(tc_packed_map[0]) == sizeof(CUtensorMap), "tensor map storage size");
-    for (int at = 1; at <= 2; ++at)
-        if (int rc = make_tensor_map_2d_bytes(reinterpret_cast<CUtensorMap*>(&tc_packed_map[at - 1]), packed,
-                                              uint64_t(geo.strips_padded), geo.strip_bytes(), geo.strip_bytes(),
-                                              kTcChunkBytes, 8 * at))
-            return rc;
-    GB_CUDA(cudaFuncSetAttribute(w4a16_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcSmem<1>::total));
-    GB_CUDA(cudaFuncSetAttribute(w4a16_tc_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcSmem<2>::total));
+    static_assert(sizeof(tc_packed_map) == sizeof(CUtensorMap), "tensor map storage size");
+    if (int rc = make_tensor_map_2d_bytes(reinterpret_cast<CUtensorMap*>(&tc_packed_map), packed, uint64_t(geo.strips_padded),
+                                          geo.strip_bytes(), geo.strip_bytes(), kTcChunkBytes, 8))
+        return rc;
+    GB_CUDA(cudaFuncSetAttribute(w4a16_tc_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcSmem::total(kTcMaxRows)));
+    GB_CUDA(cudaFuncSetAttribute(w4a16_tc_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcSmem::total(kTcHalfRows)));
     return GARNET_B200_OK;
 }
 
-int W4A16::launch_tc(const __nv_bfloat16* x, __nv_bfloat16* y, int m, void* ws, size_t ws_bytes, unsigned flags, cudaStream_t stream)
+int W4A16::launch_tc(const __nv_bfloat16* x, __nv_bfloat16* y, int m, unsigned flags, cudaStream_t stream)
 {
+    const TcPlan plan = tc_plan(geo, m);
     CUtensorMap map;
-    if (int rc = make_tensor_map_2d_16bit(&map, x, uint64_t(m), uint64_t(geo.cols), kTcTokens)) return rc;
+    if (int rc = make_tensor_map_2d_16bit(&map, x, uint64_t(m), uint64_t(geo.cols), uint32_t(plan.tile_rows))) return rc;
     TcParams p;
     p.packed = packed;
     p.y = y;
     p.fault = fault_dev;
     p.m = m;
     p.n = geo.rows;
-    p.k = geo.cols;
     p.ldy = geo.rows;
-    p.strips_padded = geo.strips_padded;
     p.chunks = geo.chunks;
-    const TcPlan plan = tc_plan(geo, m);
-    p.token_tiles = plan.token_tiles;
-    p.scale_dtype = scale_dtype;
-    const int atiles = plan.atiles;
     p.panels = plan.panels;
-    // K slices need the caller's workspace for their partial sums; without one the tiles keep all of K
-    const bool sliced = plan.kslices > 1 && ws && ws_bytes >= plan.workspace && (reinterpret_cast<uintptr_t>(ws) & 15) == 0;
-    p.kslices = sliced ? plan.kslices : 1;
-    p.chunks_per_slice = sliced ? plan.chunks_per_slice : geo.chunks;
-    p.partial = sliced ? static_cast<float*>(ws) : nullptr;
+    p.row_tiles = plan.row_tiles;
+    p.tile_rows = plan.tile_rows;
+    p.kslices = plan.kslices;
+    p.chunks_per_slice = plan.chunks_per_slice;
+    p.scale_dtype = scale_dtype;
+    const long long items = (long long)p.panels * p.row_tiles * p.kslices;
+    const bool half = items <= kSmCount && p.tile_rows <= kTcHalfRows;
+    p.tmem_cols = half ? 256 : 512;
+    p.col_a = half ? kTcHalfRows : 2 * kTcMaxRows;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(unsigned(std::min(p.panels * p.token_tiles * p.kslices, kSmCount)));
-    cfg.blockDim = dim3(tc_threads(atiles));
-    cfg.dynamicSmemBytes = atiles == 2 ? TcSmem<2>::total : TcSmem<1>::total;
+    // with K slices every CTA has one item (tc_plan keeps them below the SM count), else the CTAs are persistent
+    cfg.gridDim = dim3(unsigned(std::min<long long>(items, kSmCount)));
+    const auto kernel = half ? w4a16_tc_kernel<2> : w4a16_tc_kernel<4>;
+    cfg.blockDim = dim3(half ? tc_threads(2) : tc_threads(4));
+    cfg.dynamicSmemBytes = unsigned(TcSmem::total(p.tile_rows));
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = (flags & 1u) ? 1 : 0;
-    if (atiles == 2)
-        GB_CUDA(cudaLaunchKernelEx(&cfg, w4a16_tc_kernel<2>, p, map, *reinterpret_cast<const CUtensorMap*>(&tc_packed_map[1])));
-    else
-        GB_CUDA(cudaLaunchKernelEx(&cfg, w4a16_tc_kernel<1>, p, map, *reinterpret_cast<const CUtensorMap*>(&tc_packed_map[0])));
-    if (sliced) {
-        const size_t quads = (size_t(m) * geo.rows + 3) / 4;
-        cudaLaunchConfig_t rc = {};
-        rc.gridDim = dim3(unsigned((quads + 255) / 256));
-        rc.blockDim = dim3(256);
-        rc.stream = stream;
-        rc.attrs = attr;
-        rc.numAttrs = 1;   // starts while the tile kernel drains; waits for its results on the device
-        GB_CUDA(cudaLaunchKernelEx(&rc, w4a16_splitk_reduce_kernel, (const float*)p.partial, y, m, geo.rows, geo.rows, p.kslices));
+    cudaLaunchAttribute attr[2];
+    int attrs = 0;
+    if (p.kslices > 1) {
+        attr[attrs].id = cudaLaunchAttributeClusterDimension;
+        attr[attrs++].val.clusterDim = {unsigned(p.kslices), 1, 1};
     }
+    if (flags & 1u) {
+        attr[attrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[attrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = unsigned(attrs);
+    GB_CUDA(cudaLaunchKernelEx(&cfg, kernel, p, map, *reinterpret_cast<const CUtensorMap*>(&tc_packed_map)));
     return GARNET_B200_OK;
 }
 

@@ -103,6 +103,22 @@ def test_linear_tensor_core_tiles(n, k, m):
     check_close(y, case["x_f32"].astype(np.float64) @ wq.T)
 
 
+@pytest.mark.parametrize("scale_dtype", ["bf16", "fp16"])
+@pytest.mark.parametrize("m", [17, 31, 48, 77, 191, 192, 193, 385])
+@pytest.mark.parametrize("n,k", [(128, 128), (201, 256), (1000, 1152), (1024, 2048), (3000, 512)])
+def test_tile_kernel_shares_of_the_batch_and_of_k(n, k, m, scale_dtype):
+    """Even shares of the batch (one to three tiles, odd rows), weight rows that end inside a panel, an odd row pitch, one to
+    eight K slices with an uneven last one, both scale types."""
+    case = synth.int4_linear(n, k, m, seed=m + n + k)
+    scales = torch.from_numpy(case["scales_f32"]).reshape(n, k // 128).to(torch.float16 if scale_dtype == "fp16" else torch.bfloat16)
+    lin = garnet_b200.W4A16Linear().prepare(torch.from_numpy(case["nibbles"]).cuda(), scales.cuda(), n, k)
+    y = lin.forward(bf16_tensor(case["x_bits"]).reshape(m, k))
+    torch.cuda.synchronize()
+    assert lin.fault() == 0
+    wq = oracle.bf16_round(oracle.int4_dequant(case["nibbles"], scales.float().numpy().reshape(-1), n, k, 128)).astype(np.float64)
+    check_close(y, case["x_f32"].astype(np.float64) @ wq.T)
+
+
 def test_tile_kernel_with_and_without_k_slices():
     """More than 16 rows on a small matrix: with the workspace garnet_b200_w4a16_workspace asks
     for, K is cut into slices whose fp32 partial sums are added in slice order; without one K
