@@ -11,24 +11,27 @@
 //   MMA warp          one thread: P V of these keys when their P is there, then Q K^T of the keys two steps on into the
 //                     columns that P leaves, tile by tile: scores are ready before the softmax wants them;
 //   2 x 4 softmax     one thread per query row: 64 scores into registers, running maximum (the sink is its first value),
-//   warps             p = 2^(s c - m c), the row's sum in fp32, P over the scores in tensor memory; O in tensor memory is
-//                     rescaled only when a row's maximum has grown by more than 2^8 since the last time (the final division
-//                     makes that exact).  The fp32 work runs two values per instruction (f32x2).
+//   warps             p = 2^(s c - m c), the row's sum in fp32, P over the scores in tensor memory; the P V of the step before
+//                     is added to O, which stays in registers and is rescaled only when a row's maximum has grown by more than
+//                     2^8 since the last time (the final division makes that exact).  The fp32 work runs two values per
+//                     instruction (f32x2).
 // Numerics: the queries are bf16-valued fp32 (a tile that holds others takes the fp32 row loop instead), so Q K^T has exact
-// products.  P is fp32: it enters the MMA as two bf16 numbers, hi = bf16(p) and lo = bf16(p - hi), which leaves at most
-// 2^-18 p - less than the rounding errors of an fp32 sum over some hundreds of positions, and 2^-9 of the step of the
-// bf16 result.  A row that comes out NaN (infinities in the cache meet a zero piece) is computed again by the row loop.
+// products.  P is fp32 and enters the MMA as three bf16 numbers, which hold eight of its 24 bits each.  The tensor core truncates
+// what it accumulates, so a sum that stays in it loses about half a unit of its last place per MMA: each step starts a new one,
+// smallest pieces first, and the steps are added in fp32.  Share of the results that are not the bf16 rounding of the float64
+// result, 2048 tokens / 64 tokens after 4000: 4.2e-4 / 8.5e-4 by the fp32 row loop, 2.7e-3 / 5.2e-3 with two pieces and O in
+// tensor memory, 1.9e-3 / 6.8e-3 with three, 1.6e-4 / 2.0e-4 as it is now.  A row that comes out NaN (infinities in the cache
+// meet a zero piece) is computed again by the row loop.
 //
-// Bound: per 128 x 64 scores the tensor pipe needs about 460 clocks (8 P V MMAs at 33, 4 Q K^T MMAs at 50) and the exponentials
-// 512 (16 per clock and SM); a pair of tiles takes about 2000 per step, most of it in the instruction issue of the schedulers
-// that a loader or the MMA warp shares with two softmax warps.
-// 2048 tokens, 64 / 8 heads (ncu): 171 us with steps of 128 keys, one set of scores and the next Q K^T behind P V (6050 clocks
-// per 128 keys and pair of tiles, of which the softmax had 2300) -> 119 us.
+// Bound: per 128 x 64 scores the tensor pipe needs about 600 clocks (12 P V MMAs at 33, 4 Q K^T MMAs at 50) and the exponentials
+// 512 (16 per clock and SM); most of a step's time goes into the instruction issue of the schedulers that a loader or the MMA warp
+// shares with two softmax warps.
+// 2048 tokens, 64 / 8 heads (events, append included): 132 us; 110 us with two pieces of P and O in tensor memory, whose sums
+// were worse than the row loop's; pieces rounded instead of cut off 135 us, stored 32 keys at a time 141 us.
 #include <algorithm>
 #include <cfloat>
 
 #include "gpt_oss_attn.cuh"
-#include "mx_common.cuh"
 #include "tc_common.cuh"
 
 namespace gb200 {
@@ -40,11 +43,11 @@ constexpr int kPfKeys = 64;           // keys of a step (UMMA N of Q K^T, K of P
 constexpr int kPfStages = 8, kPfAhead = 3;
 constexpr int kPfTileBytes = 128 * 128;          // a tile of queries
 constexpr int kPfKvBytes = kPfKeys * 128;        // a step's K rows, and its V rows
-// 8 softmax warps, MMA, 2 loaders: 11 warps leave a thread 168 registers (13 would leave 128, and the softmax would spill)
+// 8 softmax warps, MMA, 2 loaders: 11 warps leave a thread 168 registers, which the softmax needs (13 would leave 128)
 constexpr int kPfMmaWarp = 8, kPfFirstLoader = 9, kPfLoaders = 2;
 constexpr int kPfThreads = (kPfFirstLoader + kPfLoaders) * 32;
-// Tensor memory of a tile: two sets of 64 scores (the hi and lo halves of P replace them), the output.
-constexpr uint32_t kPfColLo = 32, kPfColO = 128, kPfCols = 256;
+// Tensor memory of a tile: two sets of 64 scores (the first two pieces of P replace them), P V of a step, the third pieces of P.
+constexpr uint32_t kPfColMid = 32, kPfColPv = 128, kPfColLow = 192, kPfCols = 256;
 
 struct PfSmem {
     static constexpr int q = 0;                                    // [2] tiles
@@ -87,14 +90,14 @@ __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint32
         "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(uint32_t(accumulate)), "n"(kPfDescHi)
         : "memory");
 }
-__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16])
+__device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const uint32_t (&r)[8])
 {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
-        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
-        "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-        : "memory");
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+                 "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
 }
+// The upper halves of two fp32 numbers: their first eight bits, as bf16.
+__device__ __forceinline__ uint32_t upper_halves(float lo, float hi) { return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632); }
 __device__ __forceinline__ float max3(float a, float b, float c)
 {
     float r;
@@ -121,6 +124,12 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // Bits [lo, hi) of a 32-bit word, for any lo and hi.
@@ -143,9 +152,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
     uint64_t* kv_empty = kv_full + kPfStages;                               // [stages]
     uint64_t* s_full = kv_empty + kPfStages;                                // [2 tiles][2 sets] scores written
     uint64_t* p_full = s_full + 4;                                          // [2 tiles][2 sets] P written
-    uint64_t* o_full = p_full + 4;                                          // [2 tiles] P V of a step done
-    uint64_t* o_done = o_full + 2;                                          // [2 tiles] the last P V done
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 2);
+    uint64_t* pv_full = p_full + 4;                                         // [2 tiles] P V of a step done
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_full + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
@@ -163,7 +171,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
         for (int s = 0; s < 4; ++s) {
             mbar_init(&s_full[s], 1);
             mbar_init(&p_full[s], 4);
-            if (s < 2) mbar_init(&o_full[s], 1), mbar_init(&o_done[s], 1);
+            if (s < 2) mbar_init(&pv_full[s], 1);
         }
         *abort_flag = 0;
         fence_barrier_init();
@@ -298,13 +306,14 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
                     if (good && q == 0 && j + 2 < steps) good = mbar_wait_suspended(&kv_full[(j + 2) % kPfStages], ((j + 2) / kPfStages) & 1);
                     if (!good) break;
                     tc_fence_after();
-                    const uint32_t d = tmem_base + q * kPfCols + kPfColO, a = tmem_base + q * kPfCols + (j & 1) * kPfKeys;
+                    const uint32_t tile = tmem_base + q * kPfCols, set = (j & 1) * kPfKeys;
+                    const uint32_t pieces[3] = {tile + kPfColLow + set / 2, tile + set + kPfColMid, tile + set};
 #pragma unroll
-                    for (int half = 0; half < 2; ++half)
+                    for (int piece = 0; piece < 3; ++piece)
 #pragma unroll
                         for (int k16 = 0; k16 < kPfKeys / 16; ++k16)
-                            umma_ts(d, a + half * kPfColLo + k16 * 8, v + k16 * (2048 >> 4), idesc_pv, j > 0 || half > 0 || k16 > 0);
-                    umma_commit(j + 1 < steps ? &o_full[q] : &o_done[q]);
+                            umma_ts(tile + kPfColPv, pieces[piece] + k16 * 8, v + k16 * (2048 >> 4), idesc_pv, piece > 0 || k16 > 0);
+                    umma_commit(&pv_full[q]);
                     if (j + 2 < steps) scores(j + 2, q);
                 }
                 umma_commit(&kv_empty[j % kPfStages]);
@@ -325,6 +334,23 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
         const float c = 0.125f * kLog2e;                       // 1 / sqrt(64), in powers of two
         float ref = mine ? p.sinks[head] * kLog2e : 0.f;       // what the exponents are taken against
         float sum = 1.f;                                       // the sink's own term
+        uint64_t o2[kOssDim / 2];                              // O, two values each
+#pragma unroll
+        for (int i = 0; i < kOssDim / 2; ++i) o2[i] = 0;
+        // adds P V of step j
+        const auto add_pv = [&](int j) {
+            if (!mbar_wait_suspended(&pv_full[q], j & 1)) *abort_flag = 1;
+            tc_fence_after();
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                uint32_t pv[32];
+                tmem_ld_32x32(tm + kPfColPv + 32 * h, pv);
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                    o2[16 * h + i] = add2(o2[16 * h + i], f32x2(__uint_as_float(pv[2 * i]), __uint_as_float(pv[2 * i + 1])));
+            }
+        };
         for (int j = 0; j < steps && !*abort_flag; ++j) {
             const int st = j % kPfStages, kb = key0 + j * kPfKeys;
             const uint32_t ts = tm + (j & 1) * kPfKeys;
@@ -351,79 +377,75 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
             for (int i = 0; i < 32; ++i) m[i & 3] = max3(m[i & 3], __uint_as_float(s[0][i]), __uint_as_float(s[1][i]));
             const float top = fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3])) * c;
             const bool grow = j == 0 ? top > ref : top > ref + 8.f;
-            if (__any_sync(0xffffffffu, grow)) {
-                const float f = grow ? ex2(ref - top) : 1.f;
-                if (grow) ref = top;
-                sum *= f;
-                if (j > 0) {
-                    // P V of the step before has to be in O (P V of step j - 2 was done before these scores)
-                    if (!mbar_wait_suspended(&o_full[q], (j - 1) & 1)) *abort_flag = 1;
-                    tc_fence_after();
-#pragma unroll 1
-                    for (int h = 0; h < 4; ++h) {
-                        uint32_t o[16];
-                        tmem_ld_32x16(tm + kPfColO + 16 * h, o);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f);
-                        tmem_st_32x16(tm + kPfColO + 16 * h, o);
-                    }
-                }
-            }
+            const bool rescale = __any_sync(0xffffffffu, grow);
+            const float f = grow ? ex2(ref - top) : 1.f;
+            if (grow) ref = top;
+            sum *= f;
             const float base = ref == -INFINITY ? 0.f : ref;
             const uint64_t scale2 = f32x2(c, c), base2 = f32x2(-base, -base), minus1 = f32x2(-1.f, -1.f);
             uint64_t part2[2] = {0, 0};
 #pragma unroll
-            for (int w = 0; w < 2; ++w) {
-                uint32_t hi[16], lo[16];
+            for (int w = 0; w < 4; ++w) {   // 16 keys at a time
+                uint64_t e2[8];
+                uint32_t b[8];
 #pragma unroll
-                for (int i = 0; i < 16; ++i) {
+                for (int i = 0; i < 8; ++i) {
+                    const uint32_t* two = s[w >> 1] + (w & 1) * 16 + 2 * i;
                     float a, d;
-                    f32x2_split(fma2(f32x2(__uint_as_float(s[w][2 * i]), __uint_as_float(s[w][2 * i + 1])), scale2, base2), a, d);
+                    f32x2_split(fma2(f32x2(__uint_as_float(two[0]), __uint_as_float(two[1])), scale2, base2), a, d);
                     a = ex2(a), d = ex2(d);
-                    const uint64_t e2 = f32x2(a, d);
-                    part2[i & 1] = add2(part2[i & 1], e2);
-                    hi[i] = bf16x2_of(a, d);
-                    float la, ld;
-                    f32x2_split(fma2(f32x2(__uint_as_float(hi[i] << 16), __uint_as_float(hi[i] & 0xffff0000u)), minus1, e2), la, ld);
-                    lo[i] = bf16x2_of(la, ld);
+                    e2[i] = f32x2(a, d);
+                    part2[i & 1] = add2(part2[i & 1], e2[i]);
+                    b[i] = upper_halves(a, d);
                 }
-                tmem_st_32x16(ts + 16 * w, hi);
-                tmem_st_32x16(ts + kPfColLo + 16 * w, lo);
+                tmem_st_32x8(ts + 8 * w, b);
+#pragma unroll
+                for (int piece = 1; piece < 3; ++piece) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        float a, d;
+                        f32x2_split(e2[i], a, d);
+                        e2[i] = fma2(f32x2(__uint_as_float(__float_as_uint(a) & 0xffff0000u), __uint_as_float(__float_as_uint(d) & 0xffff0000u)), minus1, e2[i]);
+                        f32x2_split(e2[i], a, d);
+                        b[i] = upper_halves(a, d);
+                    }
+                    tmem_st_32x8(piece == 1 ? ts + kPfColMid + 8 * w : tm + kPfColLow + (j & 1) * (kPfKeys / 2) + 8 * w, b);
+                }
             }
             float part[2];
             f32x2_split(add2(part2[0], part2[1]), part[0], part[1]);
             sum += part[0] + part[1];
+            if (j > 0) add_pv(j - 1);   // before this step's P V takes its place
+            if (rescale) {
+                const uint64_t f2 = f32x2(f, f);
+#pragma unroll
+                for (int i = 0; i < kOssDim / 2; ++i) o2[i] = mul2(o2[i], f2);
+            }
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&p_full[q * 2 + (j & 1)]);
         }
-        if (!*abort_flag && !mbar_wait_suspended(&o_done[q], 0)) *abort_flag = 1;
-        tc_fence_after();
+        if (!*abort_flag) add_pv(steps - 1);
         // a wait that gave up leaves NaNs, which no caller can take for a result
         if (*abort_flag) sum = NAN;
         float* out = p.out + (size_t(b) * p.tokens + t) * p.q_heads * kOssDim + head * kOssDim;
         bool bad = false;
+        if (mine) {
 #pragma unroll
-        for (int h = 0; h < 4; ++h) {
-            uint32_t o[16];
-            tmem_ld_32x16(tm + kPfColO + 16 * h, o);
-            tmem_ld_wait();
-            if (mine) {
+            for (int i = 0; i < kOssDim / 4; ++i) {
+                float v[4];
+                f32x2_split(o2[2 * i], v[0], v[1]);
+                f32x2_split(o2[2 * i + 1], v[2], v[3]);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    float v[4];
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        v[e] = end > begin ? bf16_round_f(__uint_as_float(o[4 * i + e]) / sum) : 0.f;
-                        bad = bad || isnan(v[e]);
-                    }
-                    *reinterpret_cast<float4*>(out + 16 * h + 4 * i) = make_float4(v[0], v[1], v[2], v[3]);
+                for (int e = 0; e < 4; ++e) {
+                    v[e] = end > begin ? bf16_round_f(v[e] / sum) : 0.f;
+                    bad = bad || isnan(v[e]);
                 }
+                *reinterpret_cast<float4*>(out + 4 * i) = make_float4(v[0], v[1], v[2], v[3]);
             }
-            __syncwarp();
         }
+        __syncwarp();
         for (uint32_t redo = __ballot_sync(0xffffffffu, bad && !*abort_flag); redo; redo &= redo - 1) {
             const int from = __ffs(redo) - 1;
             oss_attention_row(p, __shfl_sync(0xffffffffu, b * p.tokens + t, from), __shfl_sync(0xffffffffu, head, from), lane);

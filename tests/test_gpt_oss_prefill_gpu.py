@@ -135,3 +135,20 @@ def test_infinite_values_stay_infinite():
     assert bool((got[:, :8, 7] == math.inf).all()) and bool((got[:, 8:16, 9] == -math.inf).all())
     rest = torch.isfinite(w)
     assert torch.equal(torch.isfinite(got), rest) and float((got - w)[rest].abs().max()) < 2e-2
+
+
+def test_probabilities_keep_their_24_bits():
+    """Each row sees two keys whose scores differ by d, with values 1 and -1: the result is tanh(d / 2), the difference of two
+    nearly equal probabilities, which shows what of them is left out.  Scores are single exact products; an exponential is good
+    to 2^-22 and the result is rounded to bf16 once."""
+    c = make(200, [0], 2, seed=7)
+    g = torch.Generator().manual_seed(7)
+    qkv = torch.zeros(200, 80, 64)
+    qkv[:, :64, 3] = bf(1 + torch.rand(200, 64, generator=g))
+    qkv[:, 64:72, 3] = 0.125 + torch.randint(0, 32, (200, 8), generator=g) * 2.0 ** -10
+    qkv[:, 72:, :] = (1 - 2.0 * (torch.arange(200) % 2)).reshape(-1, 1, 1)
+    c["qkv"] = qkv.reshape(200, -1).cuda()
+    c["sinks"][:] = -math.inf
+    got = run(c).to(D)
+    w, _ = want(c)
+    assert bool(((got - w).abs() <= 1.01 * 2.0 ** -8 * w.abs() + 2.0 ** -22).all()), float((got - w).abs().max())
