@@ -7,8 +7,11 @@
 // maximum and sum in fp32.  The warps of a CTA meet in shared memory, the CTAs of the cluster through distributed shared
 // memory, where each CTA finishes some of the heads: no partial results in global memory, no counter, no last CTA.
 // Numerics: K is bf16 and the queries are bf16-valued (products exact); queries that are not enter as three bf16 numbers.
-// P is fp32 and enters as three bf16 numbers (24 bits).  A row whose result is NaN (infinities in the cache meet the zero
-// pieces) is computed again by the general row loop.
+// P is fp32 and enters as three bf16 numbers (24 bits).  The tensor core truncates what it accumulates, so sums run over the
+// smallest pieces first and P V over one tile only, the tiles being added in fp32.  Share of the results that are not the bf16
+// rounding of the float64 result, 16 sequences of 8191 positions: 2.9e-4 by scalar fp32 products over splits of 64, 6.4e-4 with O
+// in the MMAs' accumulators, 1.8e-4 as it is now; queries that are not bf16 values, 3000 positions: 4.2e-4, 5.4e-4, 2.1e-4.
+// A row whose result is NaN (infinities in the cache meet the zero pieces) is computed again by the general row loop.
 //
 // Bound: the latency of its chain (lengths -> page -> rows -> softmax -> merge) at one sequence, HBM for a batch: 8 sequences
 // of 8192 positions read 134 MB.  Against scalar fp32 products over shared-memory rows with the splits merged by a last CTA:
@@ -48,7 +51,8 @@ __device__ __forceinline__ uint32_t take_piece(float& a, float& b)
     return r;
 }
 
-__global__ void __launch_bounds__(kDecMaxWarps * 32) oss_attention_decode_kernel(const OssAttn p)
+// 168 registers: three CTAs of four warps on an SM.
+__global__ void __maxnreg__(168) oss_attention_decode_kernel(const OssAttn p)
 {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ float cta_max[kDecHeads], cta_sum[kDecHeads];
@@ -133,19 +137,14 @@ __global__ void __launch_bounds__(kDecMaxWarps * 32) oss_attention_decode_kernel
 #pragma unroll
             for (int i = 0; i < 4; ++i) s[nt][i] = 0.f;
             const int row = nt * 8 + (lane & 7);
+            uint32_t kb[2][4];
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                uint32_t kb[4];
-                ldmatrix_x4(kt + row * 128 + (((half * 4 + (lane >> 3)) ^ (row & 7)) << 4), kb);
-                mma_bf16_16816(s[nt], qa[0][half * 2], kb[0], kb[1], s[nt]);
-                mma_bf16_16816(s[nt], qa[0][half * 2 + 1], kb[2], kb[3], s[nt]);
-                if (whole) {
+            for (int half = 0; half < 2; ++half) ldmatrix_x4(kt + row * 128 + (((half * 4 + (lane >> 3)) ^ (row & 7)) << 4), kb[half]);
 #pragma unroll
-                    for (int piece = 1; piece < 3; ++piece) {
-                        mma_bf16_16816(s[nt], qa[piece][half * 2], kb[0], kb[1], s[nt]);
-                        mma_bf16_16816(s[nt], qa[piece][half * 2 + 1], kb[2], kb[3], s[nt]);
-                    }
-                }
+            for (int piece = 2; piece >= 0; --piece) {
+                if (piece > 0 && !whole) continue;
+#pragma unroll
+                for (int k16 = 0; k16 < 4; ++k16) mma_bf16_16816(s[nt], qa[piece][k16], kb[k16 >> 1][(k16 & 1) * 2], kb[k16 >> 1][(k16 & 1) * 2 + 1], s[nt]);
             }
 #pragma unroll
             for (int i = 0; i < 4; ++i) s[nt][i] = (ok >> (nt * 8 + 2 * t + (i & 1))) & 1 ? s[nt][i] * scale : -INFINITY;
@@ -181,11 +180,14 @@ __global__ void __launch_bounds__(kDecMaxWarps * 32) oss_attention_decode_kernel
             const int row = lane & 15;
             uint32_t vb[4];
             ldmatrix_x4_trans(vt + row * 128 + (((d + (lane >> 4)) ^ (row & 7)) << 4), vb);
+            float pv[2][4] = {};
 #pragma unroll
             for (int piece = 2; piece >= 0; --piece) {
-                mma_bf16_16816(acc[d], pa[piece], vb[0], vb[1], acc[d]);
-                mma_bf16_16816(acc[d + 1], pa[piece], vb[2], vb[3], acc[d + 1]);
+                mma_bf16_16816(pv[0], pa[piece], vb[0], vb[1], pv[0]);
+                mma_bf16_16816(pv[1], pa[piece], vb[2], vb[3], pv[1]);
             }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[d][i] += pv[0][i], acc[d + 1][i] += pv[1][i];
         }
         __syncwarp();   // the stage is read: its next tile may come in
         request(tile + kDecStages * stride, stage, next, stage & 1);

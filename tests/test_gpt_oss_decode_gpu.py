@@ -73,3 +73,15 @@ def test_rope_access_widths_agree():
         positions = torch.randint(0, 9000, (tokens,), device="cuda")
         moved = torch.empty(x.numel() + 1, device="cuda")[1:].view_as(x).copy_(x)
         assert torch.equal(go.rope(opt, x, positions), go.rope(opt, moved, positions))
+
+
+@pytest.mark.parametrize("starts,exact,share", [([8190 - i for i in range(16)], True, 4e-4), ([2999, 2500, 2300, 2700] * 4, False, 4.7e-4)])
+def test_long_sums_round_as_fp32_sums_do(starts, exact, share):
+    """The share of results that are not the bf16 rounding of the float64 result.  Scalar fp32 sums over splits of 64 positions
+    leave 2.9e-4 and 4.2e-4 here (of 393216 results, so give or take 4e-5); accumulators that truncate 6.4e-4 and 5.4e-4."""
+    wrong = []
+    for seed in range(6):
+        c = decode(starts, 0, exact=exact, seed=seed)
+        got, (w, _) = run(c).to(D), want(c)
+        wrong.append(float((got - w.float().to(torch.bfloat16).to(D)).abs().gt(0).double().mean()))
+    assert sum(wrong) / len(wrong) < share, wrong
