@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
         // a wait that gave up leaves NaNs, which no caller can take for a result
         if (*abort_flag) sum = NAN;
         float* out = p.out + (size_t(b) * p.tokens + t) * p.q_heads * kOssDim + head * kOssDim;
-        bool bad = false;
+        bool bad = mine && ref == INFINITY;   // an infinite sink: the row loop says what comes of it
         if (mine) {
 #pragma unroll
             for (int i = 0; i < kOssDim / 4; ++i) {

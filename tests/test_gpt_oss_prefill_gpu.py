@@ -152,3 +152,14 @@ def test_probabilities_keep_their_24_bits():
     got = run(c).to(D)
     w, _ = want(c)
     assert bool(((got - w).abs() <= 1.01 * 2.0 ** -8 * w.abs() + 2.0 ** -22).all()), float((got - w).abs().max())
+
+
+def test_an_infinite_sink_gives_what_the_row_loop_gives():
+    """exp(inf - inf) is NaN for the heads with the infinite sink; the others are not touched by it."""
+    c = make(40, [100], 0, seed=6)
+    c["sinks"][5] = math.inf
+    got, (w, vmax) = run(c).to(D).reshape(40, 64, 64), want(c)
+    w = w.reshape(40, 64, 64)
+    assert bool(got[:, 5].isnan().all())
+    rest = torch.arange(64, device="cuda") != 5
+    assert bool(((got - w)[:, rest].abs() <= 1.01 * 2.0 ** -7 * w[:, rest].abs() + 2e-5 * vmax).all())
