@@ -8,6 +8,7 @@
 #include <cstdio>
 
 #include "../../include/garnet_b200.h"
+#include "launch_plan.h"
 
 namespace gb200 {
 
@@ -20,8 +21,6 @@ int cuda_fail(cudaError_t e, const char* where);
         cudaError_t e__ = (expr);                                 \
         if (e__ != cudaSuccess) return gb200::cuda_fail(e__, #expr); \
     } while (0)
-
-constexpr int kSmCount = 148;
 
 #if defined(__CUDACC__)
 

@@ -1,0 +1,46 @@
+// How launches are cut into CTAs: plain host arithmetic, without CUDA headers.
+#pragma once
+#include <algorithm>
+
+namespace gb200 {
+
+constexpr int kSmCount = 148;
+
+// Tiling of the int4 tile kernel (w4a16_tc.cu) for a batch of m rows.
+constexpr int kTcMaxRows = 192;    // batch rows per tile (UMMA N): two accumulators and four A tiles fill 512 columns
+constexpr int kTcMaxSlices = 8;    // CTAs of a cluster
+struct TcPlan {
+    int panels, row_tiles, tile_rows, kslices;
+};
+
+// The chunks of K that slice `slice` of `slices` takes are [tc_first_chunk(slice), tc_first_chunk(slice + 1)): even shares, none
+// of them empty as long as there are as many chunks as slices.  (Shares of equal length but for the last left the K of every
+// second matrix in one slice: 64 rows x 5376 -> 512 took 28.5 us, 8.2 us in eight slices of 5 or 6 chunks; any number of slices up
+// to eight instead of a power of two took 0.88 to 1.06 times as long on 35 shapes, and 23.6 instead of 15.3 us for
+// 100 x 5888 -> 3000.)
+#if defined(__CUDACC__)
+__host__ __device__
+#endif
+constexpr int tc_first_chunk(int chunks, int slices, int slice) { return slice * chunks / slices; }
+
+// As few even shares of the batch as tiles allow or, when that is more than a wave, up to three more, whichever makes the least
+// work of whole waves (an MMA costs its N columns and some fixed time, about 24 columns' worth); K slices while the machine has
+// room for twice the CTAs.
+inline TcPlan tc_plan(int strips_padded, int chunks, int m)
+{
+    TcPlan t;
+    t.panels = strips_padded / 8;
+    const int fewest = (m + kTcMaxRows - 1) / kTcMaxRows;
+    long long best = 0;
+    for (int tiles = fewest; tiles == fewest || (tiles < fewest + 4 && t.panels * fewest > kSmCount); ++tiles) {
+        const int rows = ((m + tiles - 1) / tiles + 15) / 16 * 16;
+        const long long used = (m + rows - 1) / rows, waves = (t.panels * used + kSmCount - 1) / kSmCount, cost = waves * (rows + 24);
+        if (tiles == fewest || cost < best) best = cost, t.row_tiles = int(used), t.tile_rows = rows;
+    }
+    const long long tiles = (long long)t.panels * t.row_tiles;
+    t.kslices = 1;
+    while (t.kslices < kTcMaxSlices && 2 * t.kslices <= chunks && tiles * t.kslices * 2 <= kSmCount) t.kslices *= 2;
+    return t;
+}
+
+}  // namespace gb200

@@ -40,11 +40,6 @@ struct W4A16 {
     int run(const void* d_x, void* d_y, int m, void* ws, size_t ws_bytes, unsigned flags, cudaStream_t stream);
 };
 
-// Tiling of the tensor-core tile kernel for a batch of m rows.
-struct TcPlan {
-    int panels, row_tiles, tile_rows, kslices, chunks_per_slice;
-};
-TcPlan tc_plan(const PackGeom& geo, int m);
 size_t tc_workspace(const PackGeom& geo, int m);
 
 int w4a16_repack_device(const uint8_t* d_nibbles, const uint16_t* d_scales, const PackGeom& geo, long long row0,

@@ -33,12 +33,10 @@ namespace gb200 {
 
 namespace cg = cooperative_groups;
 
-constexpr int kTcMaxRows = 192;           // batch rows per tile (UMMA N): two accumulators and four A tiles fill 512 columns
 constexpr int kTcAStages = 4;             // A tiles of 64 columns of K in tensor memory, 32 columns each
 constexpr int kTcBStages = 6;             // activation tiles of 64 columns of K
 constexpr int kTcPackStages = 4;          // packed chunks of 128 columns of K
 constexpr int kTcPrefetchChunks = 8;      // packed chunks prefetched into L2 ahead of the ring
-constexpr int kTcMaxSlices = 8;           // CTAs of a cluster
 constexpr int kTcFirstDequant = 4, kTcEpilogueWarps = 4;
 __host__ __device__ constexpr int tc_threads(int groups) { return (kTcFirstDequant + 4 * groups + kTcEpilogueWarps) * 32; }
 constexpr int kTcChunkBytes = 1024 + 32;  // int4 strip-chunk
@@ -57,7 +55,7 @@ struct TcParams {
     int ldy;
     int chunks;
     int panels, row_tiles, tile_rows;
-    int kslices, chunks_per_slice;   // the K dimension of a tile may be cut into slices handled by the CTAs of a cluster
+    int kslices;                     // the K dimension of a tile may be cut into slices handled by the CTAs of a cluster
     int scale_dtype;
     int tmem_cols, col_a;            // tensor memory: columns, and where the A tiles start
 };
@@ -74,8 +72,8 @@ __device__ __forceinline__ TcItem tc_decode(const TcParams& p, int item)
     const int rem = item - it.panel * per_panel;
     it.tt = rem / p.kslices;
     const int slice = rem - it.tt * p.kslices;
-    it.c0 = slice * p.chunks_per_slice;
-    it.c1 = min(p.chunks, it.c0 + p.chunks_per_slice);
+    it.c0 = tc_first_chunk(p.chunks, p.kslices, slice);
+    it.c1 = tc_first_chunk(p.chunks, p.kslices, slice + 1);
     return it;
 }
 
@@ -451,29 +449,6 @@ w4a16_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap x_map, con
 
 // ------------------------------------------------------------------ host side
 
-// How the tile kernel cuts the work for a batch of m rows: as few even shares of the batch as tiles allow or, when that is
-// more than a wave, up to three more, whichever makes the least work of whole waves (an MMA costs its N columns and some fixed
-// time, about 24 columns' worth); K slices while the machine has room for twice the CTAs.
-TcPlan tc_plan(const PackGeom& geo, int m)
-{
-    TcPlan t;
-    t.panels = geo.strips_padded / 8;
-    const int fewest = (m + kTcMaxRows - 1) / kTcMaxRows;
-    long long best = 0;
-    for (int tiles = fewest; tiles == fewest || (tiles < fewest + 4 && t.panels * fewest > kSmCount); ++tiles) {
-        const int rows = ((m + tiles - 1) / tiles + 15) / 16 * 16;
-        const long long used = (m + rows - 1) / rows, waves = (t.panels * used + kSmCount - 1) / kSmCount, cost = waves * (rows + 24);
-        if (tiles == fewest || cost < best) best = cost, t.row_tiles = int(used), t.tile_rows = rows;
-    }
-    const long long tiles = (long long)t.panels * t.row_tiles;
-    int slices = 1;
-    while (slices < kTcMaxSlices && 2 * slices <= geo.chunks && tiles * slices * 2 <= kSmCount) slices *= 2;
-    t.chunks_per_slice = (geo.chunks + slices - 1) / slices;
-    t.kslices = (geo.chunks + t.chunks_per_slice - 1) / t.chunks_per_slice;
-    if (t.kslices != slices) t.kslices = 1, t.chunks_per_slice = geo.chunks;   // a slice would be empty
-    return t;
-}
-
 // Workspace that a call of m rows is told to bring: fp32 partial sums of the K slices, which now meet on the chip.  The size
 // stays what callers were told before.
 size_t tc_workspace(const PackGeom& geo, int m)
@@ -545,7 +520,7 @@ int W4A16::init_tc()
 
 int W4A16::launch_tc(const __nv_bfloat16* x, __nv_bfloat16* y, int m, unsigned flags, cudaStream_t stream)
 {
-    const TcPlan plan = tc_plan(geo, m);
+    const TcPlan plan = tc_plan(geo.strips_padded, geo.chunks, m);
     CUtensorMap map;
     if (int rc = make_tensor_map_2d_16bit(&map, x, uint64_t(m), uint64_t(geo.cols), uint32_t(plan.tile_rows))) return rc;
     TcParams p;
@@ -560,7 +535,6 @@ int W4A16::launch_tc(const __nv_bfloat16* x, __nv_bfloat16* y, int m, unsigned f
     p.row_tiles = plan.row_tiles;
     p.tile_rows = plan.tile_rows;
     p.kslices = plan.kslices;
-    p.chunks_per_slice = plan.chunks_per_slice;
     p.scale_dtype = scale_dtype;
     const long long items = (long long)p.panels * p.row_tiles * p.kslices;
     const bool half = items <= kSmCount && p.tile_rows <= kTcHalfRows;

@@ -105,10 +105,11 @@ def test_linear_tensor_core_tiles(n, k, m):
 
 @pytest.mark.parametrize("scale_dtype", ["bf16", "fp16"])
 @pytest.mark.parametrize("m", [17, 31, 48, 77, 191, 192, 193, 385])
-@pytest.mark.parametrize("n,k", [(128, 128), (201, 256), (1000, 1152), (1024, 2048), (3000, 512)])
+@pytest.mark.parametrize("n,k", [(128, 128), (201, 256), (1000, 1152), (1024, 2048), (3000, 512), (201, 640), (1024, 1920), (300, 2944),
+                                 (2048, 2560), (512, 5376)])
 def test_tile_kernel_shares_of_the_batch_and_of_k(n, k, m, scale_dtype):
     """Even shares of the batch (one to three tiles, odd rows), weight rows that end inside a panel, an odd row pitch, one to
-    eight K slices with an uneven last one, both scale types."""
+    eight K slices, uneven ones (5, 9, 15, 20, 23 and 42 chunks) among them, both scale types."""
     case = synth.int4_linear(n, k, m, seed=m + n + k)
     scales = torch.from_numpy(case["scales_f32"]).reshape(n, k // 128).to(torch.float16 if scale_dtype == "fp16" else torch.bfloat16)
     lin = garnet_b200.W4A16Linear().prepare(torch.from_numpy(case["nibbles"]).cuda(), scales.cuda(), n, k)
