@@ -9,6 +9,11 @@ constexpr int kSmCount = 148;
 // Tiling of the int4 tile kernel (w4a16_tc.cu) for a batch of m rows.
 constexpr int kTcMaxRows = 192;    // batch rows per tile (UMMA N): two accumulators and four A tiles fill 512 columns
 constexpr int kTcMaxSlices = 8;    // CTAs of a cluster
+constexpr int kTcSharedRows = 96;  // the largest tile with which two CTAs share an SM's memory
+// CTAs in clusters of 2, 4 or 8 that run at once when each has an SM for itself: a cluster lies within a GPC, which has 16 or 18
+// SMs or fewer, so that less than the whole GPU is left the larger the clusters are (74, 33 and 15 of them fit a B200, by
+// cudaOccupancyMaxActiveClusters; a little less is asked for here).
+constexpr int tc_cluster_room(int slices) { return slices <= 2 ? kSmCount : slices <= 4 ? 128 : 112; }
 struct TcPlan {
     int panels, row_tiles, tile_rows, kslices;
 };
@@ -25,7 +30,8 @@ constexpr int tc_first_chunk(int chunks, int slices, int slice) { return slice *
 
 // As few even shares of the batch as tiles allow or, when that is more than a wave, up to three more, whichever makes the least
 // work of whole waves (an MMA costs its N columns and some fixed time, about 24 columns' worth); K slices while the machine has
-// room for twice the CTAs.
+// room for twice the CTAs: a cluster that has to wait for another to finish doubles the call (256 rows x 2048 -> 1024, 16
+// clusters of 8: 17.2 us; as 16 of 4: 9.3 us).
 inline TcPlan tc_plan(int strips_padded, int chunks, int m)
 {
     TcPlan t;
@@ -39,7 +45,8 @@ inline TcPlan tc_plan(int strips_padded, int chunks, int m)
     }
     const long long tiles = (long long)t.panels * t.row_tiles;
     t.kslices = 1;
-    while (t.kslices < kTcMaxSlices && 2 * t.kslices <= chunks && tiles * t.kslices * 2 <= kSmCount) t.kslices *= 2;
+    const auto room = [&](int slices) { return t.tile_rows > kTcSharedRows ? tc_cluster_room(slices) : kSmCount; };
+    while (t.kslices < kTcMaxSlices && 2 * t.kslices <= chunks && tiles * t.kslices * 2 <= room(2 * t.kslices)) t.kslices *= 2;
     return t;
 }
 

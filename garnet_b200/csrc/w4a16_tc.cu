@@ -86,6 +86,8 @@ struct TcSmem {
     static constexpr int total(int tile_rows) { return b + kTcBStages * tile_rows * 128 + 1024; }   // slack for 1024-byte alignment
 };
 static_assert(128 * 4 <= kTcBStages * 128, "partial tile");
+static_assert(2 * (TcSmem::total(kTcSharedRows) + 1024) <= 228 * 1024 && 2 * (TcSmem::total(kTcSharedRows + 16) + 1024) > 228 * 1024,
+              "tiles with which two CTAs share an SM");
 
 // One int4 word (8 codes of one row, pair-interleaved) times a scale -> 8 bf16.
 __device__ __forceinline__ uint4 int4_word_to_bf16x8(uint32_t w, uint32_t scale_bf16x2)
