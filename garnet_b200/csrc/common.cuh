@@ -102,6 +102,15 @@ __device__ __forceinline__ bool mbar_wait_suspended(uint64_t* bar, uint32_t pari
         if (global_timer_ns() - t0 > limit_ns) return false;
     return true;
 }
+// The wait of a whole warp: every lane gets the same answer, so that the warp leaves its loop together and never comes to an
+// instruction that all of its lanes have to execute with some of them gone.  A warp that gives up says so in `abort_flag` (shared
+// memory); those that wait for what it would have done give up in their turn.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, unsigned long long limit_ns = kWaitLimitNs)
+{
+    const bool all = __all_sync(0xffffffffu, mbar_wait_suspended(bar, parity, limit_ns));
+    if (!all) *abort_flag = 1;
+    return all;
+}
 __device__ __forceinline__ void fence_barrier_init()
 {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");

@@ -153,7 +153,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
     uint64_t* s_full = kv_empty + kPfStages;                                // [2 tiles][2 sets] scores written
     uint64_t* p_full = s_full + 4;                                          // [2 tiles][2 sets] P written
     uint64_t* pv_full = p_full + 4;                                         // [2 tiles] P V of a step done
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_full + 2);
+    uint64_t* drained = pv_full + 2;                                        // every MMA done
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drained + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
@@ -173,6 +174,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
             mbar_init(&p_full[s], 4);
             if (s < 2) mbar_init(&pv_full[s], 1);
         }
+        mbar_init(drained, 1);
         *abort_flag = 0;
         fence_barrier_init();
     }
@@ -262,16 +264,13 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
     if (warp >= kPfFirstLoader) {
         // -------------------------------------------------------------- loaders
         // a step is announced as soon as it is there, before the wait for the stage of the next request
-        for (int j = 0; j < steps && !*abort_flag; ++j) {
+        for (int j = 0; j < steps; ++j) {
             asm volatile("cp.async.wait_group %0;" ::"n"(kPfAhead - 1) : "memory");
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) mbar_arrive(&kv_full[j % kPfStages]);
             const int next = j + kPfAhead;
-            if (next >= kPfStages && next < steps && !mbar_wait_suspended(&kv_empty[next % kPfStages], ((next / kPfStages) - 1) & 1)) {
-                *abort_flag = 1;
-                break;
-            }
+            if (next >= kPfStages && next < steps && !mbar_wait_warp(&kv_empty[next % kPfStages], ((next / kPfStages) - 1) & 1, abort_flag)) break;
             request(next, ahead);
             ahead = look_up(next + 1);
         }
@@ -319,6 +318,9 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
                 umma_commit(&kv_empty[j % kPfStages]);
             }
             if (!good) *abort_flag = 1;
+            // no MMA is in flight when the CTA gives its memory back, also after a wait that gave up
+            umma_commit(drained);
+            mbar_wait_suspended(drained, 0);
         }
         __syncwarp();
     } else if ((warp >> 2) < qtiles) {
@@ -338,8 +340,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
 #pragma unroll
         for (int i = 0; i < kOssDim / 2; ++i) o2[i] = 0;
         // adds P V of step j
-        const auto add_pv = [&](int j) {
-            if (!mbar_wait_suspended(&pv_full[q], j & 1)) *abort_flag = 1;
+        const auto add_pv = [&](int j) -> bool {
+            if (!mbar_wait_warp(&pv_full[q], j & 1, abort_flag)) return false;
             tc_fence_after();
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
@@ -350,14 +352,14 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
                 for (int i = 0; i < 16; ++i)
                     o2[16 * h + i] = add2(o2[16 * h + i], f32x2(__uint_as_float(pv[2 * i]), __uint_as_float(pv[2 * i + 1])));
             }
+            return true;
         };
-        for (int j = 0; j < steps && !*abort_flag; ++j) {
+        bool good = true;
+        for (int j = 0; j < steps; ++j) {
             const int st = j % kPfStages, kb = key0 + j * kPfKeys;
             const uint32_t ts = tm + (j & 1) * kPfKeys;
-            if (!mbar_wait_suspended(&kv_full[st], (j / kPfStages) & 1) || !mbar_wait_suspended(&s_full[q * 2 + (j & 1)], (j >> 1) & 1)) {
-                *abort_flag = 1;
-                break;
-            }
+            good = mbar_wait_warp(&kv_full[st], (j / kPfStages) & 1, abort_flag) && mbar_wait_warp(&s_full[q * 2 + (j & 1)], (j >> 1) & 1, abort_flag);
+            if (!good) break;
             tc_fence_after();
             uint32_t s[2][32];
             tmem_ld_32x32(ts, s[0]);
@@ -415,7 +417,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
             float part[2];
             f32x2_split(add2(part2[0], part2[1]), part[0], part[1]);
             sum += part[0] + part[1];
-            if (j > 0) add_pv(j - 1);   // before this step's P V takes its place
+            good = j == 0 || add_pv(j - 1);   // before this step's P V takes its place
+            if (!good) break;
             if (rescale) {
                 const uint64_t f2 = f32x2(f, f);
 #pragma unroll
@@ -426,9 +429,9 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
             __syncwarp();
             if (lane == 0) mbar_arrive(&p_full[q * 2 + (j & 1)]);
         }
-        if (!*abort_flag) add_pv(steps - 1);
+        good = good && add_pv(steps - 1);
         // a wait that gave up leaves NaNs, which no caller can take for a result
-        if (*abort_flag) sum = NAN;
+        if (!good) sum = NAN;
         float* out = p.out + (size_t(b) * p.tokens + t) * p.q_heads * kOssDim + head * kOssDim;
         bool bad = mine && ref == INFINITY;   // an infinite sink: the row loop says what comes of it
         if (mine) {
@@ -446,7 +449,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
             }
         }
         __syncwarp();
-        for (uint32_t redo = __ballot_sync(0xffffffffu, bad && !*abort_flag); redo; redo &= redo - 1) {
+        for (uint32_t redo = __ballot_sync(0xffffffffu, bad && good); redo; redo &= redo - 1) {
             const int from = __ffs(redo) - 1;
             oss_attention_row(p, __shfl_sync(0xffffffffu, b * p.tokens + t, from), __shfl_sync(0xffffffffu, head, from), lane);
         }

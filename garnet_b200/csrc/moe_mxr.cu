@@ -161,7 +161,8 @@ moe_mxr_kernel(const RxParams p, const __grid_constant__ CUtensorMap w_map, cons
     uint64_t* empty = full + kRxStages;
     uint64_t* acc_full = empty + kRxStages;
     uint64_t* acc_empty = acc_full + 2;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    uint64_t* drained = acc_empty + 2;            // every MMA done
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drained + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
@@ -174,6 +175,7 @@ moe_mxr_kernel(const RxParams p, const __grid_constant__ CUtensorMap w_map, cons
             mbar_init(&acc_full[s], 1);
             mbar_init(&acc_empty[s], kRxEpiWarps);
         }
+        mbar_init(drained, 1);
         *abort_flag = 0;
         fence_barrier_init();
     }
@@ -254,6 +256,7 @@ moe_mxr_kernel(const RxParams p, const __grid_constant__ CUtensorMap w_map, cons
                     }
                 }
             }
+            ring_wait_landed(full, kRxStages, s, round);
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------- MMA issuer
@@ -318,6 +321,9 @@ moe_mxr_kernel(const RxParams p, const __grid_constant__ CUtensorMap w_map, cons
                 if (good) umma_commit(&acc_full[buf]);
             }
             if (!good) *abort_flag = 1;
+            // no MMA is in flight when the CTA gives its memory back, also after a wait that gave up
+            umma_commit(drained);
+            mbar_wait_suspended(drained, 0);
         }
         __syncwarp();
     } else if (warp < kRxFirstEpi) {
@@ -330,12 +336,11 @@ moe_mxr_kernel(const RxParams p, const __grid_constant__ CUtensorMap w_map, cons
         const int l = quarter * 32 + lane;   // TMEM lane = routed row of the tile
         uint32_t it_n = 0;
         int cur = 0;
-        for (int item = blockIdx.x; item < items && !*abort_flag; item += gridDim.x, ++it_n) {
+        for (int item = blockIdx.x; item < items; item += gridDim.x, ++it_n) {
             const RxItem it = rx_decode(p, tile_prefix, item, cur);
             const uint32_t buf = it_n & 1;
-            if (!mbar_wait_suspended(&acc_full[buf], (it_n >> 1) & 1)) {
-                atomicExch(p.fault, 45);
-                *abort_flag = 1;
+            if (!mbar_wait_warp(&acc_full[buf], (it_n >> 1) & 1, abort_flag)) {
+                atomicCAS(p.fault, 0, 45);
                 break;
             }
             tc_fence_after();

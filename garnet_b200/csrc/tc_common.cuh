@@ -105,6 +105,16 @@ __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint6
         : "memory");
 }
 
+// Waits for the copies of a ring that has been filled `round` times and `next` stages more: none is in flight when the CTA gives
+// its memory back, also when their reader has given up.
+__device__ __forceinline__ void ring_wait_landed(uint64_t* full, int stages, uint32_t next, uint32_t round)
+{
+    for (int s = 0; s < stages; ++s) {
+        const uint32_t fills = round + (uint32_t(s) < next);
+        if (fills) mbar_wait_suspended(&full[s], (fills - 1) & 1);
+    }
+}
+
 // Arrive on `bar` once all tcgen05.mma issued so far by this thread have completed.
 __device__ __forceinline__ void umma_commit(uint64_t* bar)
 {

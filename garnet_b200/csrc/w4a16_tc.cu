@@ -82,7 +82,7 @@ __device__ __forceinline__ TcItem tc_decode(const TcParams& p, int item)
 struct TcSmem {
     static constexpr int pk = 0;
     static constexpr int bars = pk + kTcPackStages * kTcPackBytes;
-    static constexpr int b = (bars + 256 + 1023) / 1024 * 1024;
+    static constexpr int b = (bars + 512 + 1023) / 1024 * 1024;
     static constexpr int total(int tile_rows) { return b + kTcBStages * tile_rows * 128 + 1024; }   // slack for 1024-byte alignment
 };
 static_assert(128 * 4 <= kTcBStages * 128, "partial tile");
@@ -182,7 +182,8 @@ w4a16_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap x_map, con
     uint64_t* b_empty = b_full + kTcBStages;           // [kTcBStages]
     uint64_t* acc_full = b_empty + kTcBStages;         // [2]
     uint64_t* acc_empty = acc_full + 2;                // [2]
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    uint64_t* drained = acc_empty + 2;                 // every MMA done
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drained + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
@@ -203,6 +204,7 @@ w4a16_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap x_map, con
             mbar_init(&acc_full[s], 1);
             mbar_init(&acc_empty[s], kTcEpilogueWarps);
         }
+        mbar_init(drained, 1);
         *abort_flag = 0;
         fence_barrier_init();
     }
@@ -258,6 +260,7 @@ w4a16_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap x_map, con
                     }
                 }
             }
+            ring_wait_landed(pk_full, kTcPackStages, ps, round);
         }
     } else if (warp == 2) {
         // ------------------------------------------ producer of activation tiles
@@ -278,6 +281,7 @@ w4a16_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap x_map, con
                     if (++s == kTcBStages) s = 0, ++round;
                 }
             }
+            ring_wait_landed(b_full, kTcBStages, s, round);
         }
     } else if (warp == 1) {
         // ----------------------------------------------------------- MMA issuer
@@ -316,6 +320,9 @@ w4a16_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap x_map, con
                 if (good) umma_commit(&acc_full[buf]);
             }
             if (!good) *abort_flag = 1;
+            // no MMA is in flight when the CTA gives its memory back, also after a wait that gave up
+            umma_commit(drained);
+            mbar_wait_suspended(drained, 0);
         }
     } else if (warp >= kTcFirstDequant && warp < kTcFirstEpilogue) {
         // -------------------------------------------------------------- dequant
@@ -330,15 +337,16 @@ w4a16_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap x_map, con
         const uint8_t* scales = pk_ring + strip * kTcChunkBytes + 1024 + g * 4 + (upper ? 2 : 0);
         const uint32_t a_tiles = tmem_base + (uint32_t(quarter * 32) << 16) + p.col_a;
         uint32_t n = 0;   // chunks that have gone by
-        for (int item = blockIdx.x; item < items && !*abort_flag; item += gridDim.x) {
+        bool good = true;
+        for (int item = blockIdx.x; item < items && good; item += gridDim.x) {
             const TcItem it = tc_decode(p, item);
             for (int c = it.c0; c < it.c1; ++c, ++n) {
                 if (kGroups == 4 && int(n & 1) != group >> 1) continue;
                 const uint32_t tile = 2 * (n & 1) + half;
                 const uint32_t ps = n % kTcPackStages;
-                if (!mbar_wait_suspended(&pk_full[ps], (n / kTcPackStages) & 1)) {
-                    atomicExch(p.fault, 15);
-                    *abort_flag = 1;
+                good = mbar_wait_warp(&pk_full[ps], (n / kTcPackStages) & 1, abort_flag);
+                if (!good) {
+                    atomicCAS(p.fault, 0, 15);
                     break;
                 }
                 uint32_t w[8];
@@ -358,9 +366,9 @@ w4a16_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap x_map, con
 #pragma unroll
                     for (int t = 0; t < 8; ++t) v[t] = int4_word_to_bf16x8_f32(w[t], f);
                 }
-                if (n >= 2 && !mbar_wait_suspended(&a_empty[tile], ((n >> 1) - 1) & 1)) {
-                    atomicExch(p.fault, 16);
-                    *abort_flag = 1;
+                good = n < 2 || mbar_wait_warp(&a_empty[tile], ((n >> 1) - 1) & 1, abort_flag);
+                if (!good) {
+                    atomicCAS(p.fault, 0, 16);
                     break;
                 }
                 tc_fence_after();
@@ -377,12 +385,11 @@ w4a16_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap x_map, con
         const int quarter = warp & 3;   // TMEM lanes 32*quarter .. +31 belong to this warp
         const bool wide = (p.ldy & 1) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 3) == 0, odd = lane & 1;
         uint32_t it_n = 0;
-        for (int item = blockIdx.x; item < items && !*abort_flag; item += gridDim.x, ++it_n) {
+        for (int item = blockIdx.x; item < items; item += gridDim.x, ++it_n) {
             const TcItem it = tc_decode(p, item);
             const uint32_t buf = it_n & 1;
-            if (!mbar_wait_suspended(&acc_full[buf], (it_n >> 1) & 1)) {
-                atomicExch(p.fault, 17);
-                *abort_flag = 1;
+            if (!mbar_wait_warp(&acc_full[buf], (it_n >> 1) & 1, abort_flag)) {
+                atomicCAS(p.fault, 0, 17);
                 break;
             }
             tc_fence_after();
