@@ -15,12 +15,12 @@
 //                     is added to O, which stays in registers and is rescaled only when a row's maximum has grown by more than
 //                     2^8 since the last time (the final division makes that exact).  The fp32 work runs two values per
 //                     instruction (f32x2).
-// Numerics: the queries are bf16-valued fp32 (a tile that holds others takes the fp32 row loop instead), so Q K^T has exact
-// products.  P is fp32 and enters the MMA as three bf16 numbers, which hold eight of its 24 bits each.  The tensor core truncates
-// what it accumulates, so a sum that stays in it loses about half a unit of its last place per MMA: each step starts a new one,
-// smallest pieces first, and the steps are added in fp32.  Share of the results that are not the bf16 rounding of the float64
-// result, 2048 tokens / 64 tokens after 4000: 4.2e-4 / 8.5e-4 by the fp32 row loop, 2.7e-3 / 5.2e-3 with two pieces and O in
-// tensor memory, 1.9e-3 / 6.8e-3 with three, 1.6e-4 / 2.0e-4 as it is now.  A row that comes out NaN (infinities in the cache
+// Numerics: the queries are bf16-valued fp32, so Q K^T has exact products; the queries of a CTA that holds others enter as three
+// bf16 numbers each.  P is fp32 and enters the MMA as three bf16 numbers, which hold eight of its 24 bits each.  The tensor core
+// truncates what it accumulates, so a sum that stays in it loses about half a unit of its last place per MMA: each step starts a
+// new one, smallest pieces first, and the steps are added in fp32.  Share of the results that are not the bf16 rounding of the
+// float64 result, 2048 tokens / 64 tokens after 4000: 4.2e-4 / 8.5e-4 by the fp32 row loop, 2.7e-3 / 5.2e-3 with two pieces and O
+// in tensor memory, 1.9e-3 / 6.8e-3 with three, 1.6e-4 / 2.0e-4 as it is now.  A row that comes out NaN (infinities in the cache
 // meet a zero piece) is computed again by the row loop.
 //
 // Bound: per 128 x 64 scores the tensor pipe needs about 600 clocks (12 P V MMAs at 33, 4 Q K^T MMAs at 50) and the exponentials
@@ -50,12 +50,13 @@ constexpr int kPfThreads = (kPfFirstLoader + kPfLoaders) * 32;
 constexpr uint32_t kPfColMid = 32, kPfColPv = 128, kPfColLow = 192, kPfCols = 256;
 
 struct PfSmem {
-    static constexpr int q = 0;                                    // [2] tiles
-    static constexpr int kv = q + 2 * kPfTileBytes;                // [stages] K tile, V tile
+    static constexpr int q = 0;                                    // [3 pieces][2 tiles]; the first piece alone when it says it all
+    static constexpr int kv = q + 6 * kPfTileBytes;                // [stages] K tile, V tile
     static constexpr int ok = kv + kPfStages * 2 * kPfKvBytes;     // [stages][2] bits of the keys that exist
     static constexpr int bars = ok + kPfStages * 8;
     static constexpr int total = bars + 256 + 1024;                // barriers, and slack for 1024-byte alignment
 };
+static_assert(PfSmem::total <= 227 * 1024, "shared memory budget");
 
 __device__ __forceinline__ float ex2(float x)
 {
@@ -220,6 +221,22 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    // ---- queries: 8 values of a row (zeros where there is none), and their place in a tile
+    const auto load_queries = [&](int i, float (&f)[8]) {
+        const int row = i >> 3, r = row & (kPfRows - 1), in_tile = r / group, t = t0 + (row >> 7) * tile_tokens + in_tile;
+        float4 f0 = make_float4(0.f, 0.f, 0.f, 0.f), f1 = f0;
+        if (steps && in_tile < tile_tokens && t < t1) {
+            const size_t packed = size_t(p.q_heads + 2 * p.kv_heads) * kOssDim;
+            const float4* src = reinterpret_cast<const float4*>(p.qkv + (size_t(b) * p.tokens + t) * packed + (kv * group + r % group) * kOssDim + (i & 7) * 8);
+            f0 = __ldg(src), f1 = __ldg(src + 1);
+        }
+        f[0] = f0.x, f[1] = f0.y, f[2] = f0.z, f[3] = f0.w, f[4] = f1.x, f[5] = f1.y, f[6] = f1.z, f[7] = f1.w;
+    };
+    const auto store_queries = [&](int i, int piece, const float (&f)[8]) {
+        const int row = i >> 3;
+        *reinterpret_cast<uint4*>(q_tiles + piece * 2 * kPfTileBytes + row * 128 + (((i & 7) ^ (row & 7)) << 4)) =
+            make_uint4(bf16x2_of(f[0], f[1]), bf16x2_of(f[2], f[3]), bf16x2_of(f[4], f[5]), bf16x2_of(f[6], f[7]));
+    };
     unsigned long long ahead = SIZE_MAX;   // rows of the next step to request
     int inexact = 0;
     if (warp >= kPfFirstLoader) {
@@ -229,30 +246,39 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
         ahead = look_up(kPfAhead);
     } else {
         // ---- queries: fp32 to bf16, 128-byte-swizzled K-major tiles
-        const int packed = (p.q_heads + 2 * p.kv_heads) * kOssDim;
 #pragma unroll 4
         for (int i = threadIdx.x; i < qtiles * kPfRows * 8; i += kPfFirstLoader * 32) {
-            const int row = i >> 3, piece = i & 7, r = row & (kPfRows - 1), in_tile = r / group;
-            const int t = t0 + (row >> 7) * tile_tokens + in_tile, head = kv * group + r % group;
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (steps && in_tile < tile_tokens && t < t1) {
-                const float4* src = reinterpret_cast<const float4*>(p.qkv + (size_t(b) * p.tokens + t) * packed + head * kOssDim + piece * 8);
-                const float4 f0 = __ldg(src), f1 = __ldg(src + 1);
-                const float f[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
+            float f[8];
+            load_queries(i, f);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) inexact |= int(__float_as_uint(f[j]) & 0xffffu);
-                v = make_uint4(bf16x2_of(f0.x, f0.y), bf16x2_of(f0.z, f0.w), bf16x2_of(f1.x, f1.y), bf16x2_of(f1.z, f1.w));
-            }
-            *reinterpret_cast<uint4*>(q_tiles + row * 128 + ((piece ^ (row & 7)) << 4)) = v;
+            for (int j = 0; j < 8; ++j) inexact |= int(__float_as_uint(f[j]) & 0xffffu);
+            store_queries(i, 0, f);
         }
         fence_proxy_async_smem();
     }
     tc_fence_before();
-    const bool row_loop = __syncthreads_or(inexact) || steps == 0;
+    const int q_pieces = __syncthreads_or(inexact) ? 3 : 1;
+    if (q_pieces > 1) {
+        // some query is not a bf16 value: the second and third pieces of them all
+        if (warp < kPfFirstLoader) {
+            for (int i = threadIdx.x; i < qtiles * kPfRows * 8; i += kPfFirstLoader * 32) {
+                float f[8];
+                load_queries(i, f);
+#pragma unroll
+                for (int piece = 1; piece < 3; ++piece) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) f[j] -= bf16_round_f(f[j]);
+                    store_queries(i, piece, f);
+                }
+            }
+            fence_proxy_async_smem();
+        }
+        __syncthreads();
+    }
     tc_fence_after();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
-    if (row_loop) {
-        // queries that are not bf16 values (outside the operand's contract), or no visible key at all
+    if (steps == 0) {
+        // no visible key
         const int rows = (t1 - t0) * group;
         for (int i = warp; i < rows; i += kPfThreads / 32)
             oss_attention_row(p, b * p.tokens + t0 + i / group, kv * group + i % group, lane);
@@ -286,8 +312,12 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
             const auto scores = [&](int j, int q) {
                 const uint32_t d = tmem_base + q * kPfCols + (j & 1) * kPfKeys;
                 const uint32_t a = q_lo + q * (kPfTileBytes >> 4), k = k_lo + (j % kPfStages) * kStage;
+#pragma unroll 1
+                for (int piece = q_pieces - 1; piece >= 0; --piece) {
 #pragma unroll
-                for (int k16 = 0; k16 < kOssDim / 16; ++k16) umma_ss(d, a + k16 * 2, k + k16 * 2, idesc_qk, k16 > 0);
+                    for (int k16 = 0; k16 < kOssDim / 16; ++k16)
+                        umma_ss(d, a + piece * (2 * kPfTileBytes >> 4) + k16 * 2, k + k16 * 2, idesc_qk, piece + 1 < q_pieces || k16 > 0);
+                }
                 umma_commit(&s_full[q * 2 + (j & 1)]);
             };
             bool good = true;

@@ -163,3 +163,32 @@ def test_an_infinite_sink_gives_what_the_row_loop_gives():
     assert bool(got[:, 5].isnan().all())
     rest = torch.arange(64, device="cuda") != 5
     assert bool(((got - w)[:, rest].abs() <= 1.01 * 2.0 ** -7 * w[:, rest].abs() + 2e-5 * vmax).all())
+
+
+def device_us(c, calls=5):
+    ws = torch.zeros(1 << 24, dtype=torch.uint8, device="cuda")
+    def one():
+        go.attention(c["opt"], c["qkv"], c["keys"], c["values"], c["table"], c["lengths"], c["starts"], c["active"], c["sinks"],
+                     c["batch"], c["tokens"], c["physical"], workspace=ws)
+    one()
+    best = math.inf
+    for _ in range(5):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        for _ in range(calls):
+            one()
+        b.record()
+        b.synchronize()
+        best = min(best, a.elapsed_time(b) * 1000 / calls)
+    return best
+
+
+def test_queries_that_are_not_bf16_values_stay_on_the_tensor_cores():
+    """Three pieces of each query: two tiles per block, one query alone that needs them, and no row loop over the keys (which
+    took some hundred times as long)."""
+    check(make(700, [0], 0, exact=False, seed=8))
+    c = make(300, [40], 128, seed=9)
+    c["qkv"][123, 17 * 64 + 5] += 2.0 ** -12
+    check(c)
+    plain, pieces = make(512, [0], 0, seed=10), make(512, [0], 0, exact=False, seed=10)
+    assert device_us(pieces) < 4 * device_us(plain)
