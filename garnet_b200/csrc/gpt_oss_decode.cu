@@ -109,14 +109,17 @@ __global__ void __maxnreg__(168) oss_attention_decode_kernel(const OssAttn p)
     // ---- queries: MMA row = head of the group, in bf16 pieces (one when all are bf16 values)
     uint32_t qa[3][4][4];
     uint32_t inexact = 0;
+    const bool q_pairs = (reinterpret_cast<uintptr_t>(p.qkv) & 7) == 0, out_wide = (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks)
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
             const int head = g + 8 * (r & 1), d = ks * 16 + 2 * t + 8 * (r >> 1);
             float2 f = make_float2(0.f, 0.f);
-            if (head < group)
-                f = *reinterpret_cast<const float2*>(p.qkv + size_t(b) * (p.q_heads + 2 * p.kv_heads) * kOssDim + (kv * group + head) * kOssDim + d);
+            if (head < group) {
+                const float* from = p.qkv + size_t(b) * (p.q_heads + 2 * p.kv_heads) * kOssDim + (kv * group + head) * kOssDim + d;
+                f = q_pairs ? *reinterpret_cast<const float2*>(from) : make_float2(from[0], from[1]);
+            }
             inexact |= (__float_as_uint(f.x) | __float_as_uint(f.y)) & 0xffffu;
 #pragma unroll
             for (int piece = 0; piece < 3; ++piece) qa[piece][ks][r] = take_piece(f.x, f.y);
@@ -260,8 +263,11 @@ __global__ void __maxnreg__(168) oss_attention_decode_kernel(const OssAttn p)
             if (live)
                 r = make_float4(bf16_round_f(o.x / total), bf16_round_f(o.y / total), bf16_round_f(o.z / total), bf16_round_f(o.w / total));
             bad = isnan(r.x) || isnan(r.y) || isnan(r.z) || isnan(r.w);
-            *reinterpret_cast<float4*>(p.out + (size_t(b) * p.q_heads + kv * group + head) * kOssDim + d4) = r;
+            float* to = p.out + (size_t(b) * p.q_heads + kv * group + head) * kOssDim + d4;
+            if (out_wide) *reinterpret_cast<float4*>(to) = r;
+            else to[0] = r.x, to[1] = r.y, to[2] = r.z, to[3] = r.w;
         }
+        __syncwarp();   // the row loop writes over what these lanes have written
         const uint32_t redo = __ballot_sync(0xffffffffu, bad);
         for (int h = 0; h < 2; ++h)
             if ((redo >> (16 * h)) & 0xffffu) oss_attention_row(p, b, kv * group + (h0 + h) * splits + split, lane);
@@ -273,9 +279,8 @@ __global__ void __maxnreg__(168) oss_attention_decode_kernel(const OssAttn p)
 
 bool oss_decode_takes(const OssAttn& p)
 {
-    const uintptr_t bits = reinterpret_cast<uintptr_t>(p.keys) | reinterpret_cast<uintptr_t>(p.values) | reinterpret_cast<uintptr_t>(p.out);
-    return p.tokens == 1 && !p.prefill && p.head_dim == kOssDim && p.q_heads / p.kv_heads <= kDecHeads && (bits & 15) == 0 &&
-           (reinterpret_cast<uintptr_t>(p.qkv) & 7) == 0 && p.batch <= 65535;
+    const uintptr_t bits = reinterpret_cast<uintptr_t>(p.keys) | reinterpret_cast<uintptr_t>(p.values);
+    return p.tokens == 1 && !p.prefill && p.head_dim == kOssDim && p.q_heads / p.kv_heads <= kDecHeads && (bits & 15) == 0 && p.batch <= 65535;
 }
 
 int oss_decode_launch(const OssAttn& p, cudaStream_t stream)

@@ -1,13 +1,15 @@
 """gpt-oss decode attention (gpt_oss_decode.cu) against a float64 restatement of RunGptOssAttention
 (plugins/gpt_oss/cuda/gpt_oss_kernels.cu:125-160,376-535), at the sizes where its tiles of 16 positions, rounds of
 warps and clusters can go wrong, and RoPE's two access widths against each other."""
+import ctypes
 import math
 
 import pytest
 import torch
 
 from garnet_b200 import gpt_oss as go
-from test_gpt_oss_prefill_gpu import D, check, make, run, want
+from garnet_b200._lib import check as check_code, lib
+from test_gpt_oss_prefill_gpu import D, check, device_us, make, run, want
 
 pytestmark = pytest.mark.gpu
 
@@ -59,11 +61,25 @@ def test_infinite_values_stay_infinite():
     assert torch.equal(torch.isfinite(got), rest) and float((got - w)[rest].abs().max()) < 2e-2
 
 
-def test_operands_that_are_not_aligned_take_the_row_loop():
-    c = decode([100, 33], 0, seed=6)
-    buf = torch.empty(c["qkv"].numel() + 1, device="cuda")
-    moved = buf[1:].view_as(c["qkv"]).copy_(c["qkv"])
+@pytest.mark.parametrize("shift", [1, 2, 3])
+def test_operands_aligned_to_their_values_only(shift):
+    """Queries and output at any multiple of four bytes, on the same kernel (the row loop takes some fifty times as long)."""
+    c = decode([100, 33, 3000], 0, seed=6)
+    moved = torch.empty(c["qkv"].numel() + 4, device="cuda")[shift:][:c["qkv"].numel()].view_as(c["qkv"]).copy_(c["qkv"])
     check(dict(c, qkv=moved))
+    want_y = run(c)
+    y = torch.zeros(want_y.numel() + 8, device="cuda")
+    need = ctypes.c_size_t(0)
+    logical = c["table"].shape[1]
+    check_code(lib().garnet_b200_gpt_oss_attention_workspace(ctypes.byref(c["opt"]), c["batch"], logical, ctypes.byref(need)))
+    ws = torch.zeros(need.value, dtype=torch.uint8, device="cuda")
+    operands = (ctypes.c_void_p * 8)(*[t.data_ptr() for t in (moved, c["keys"], c["values"], c["table"], c["lengths"], c["starts"],
+                                                              c["active"], c["sinks"])])
+    check_code(lib().garnet_b200_gpt_oss_attention(ctypes.byref(c["opt"]), operands, y.data_ptr() + 4 * shift, ws.data_ptr(), ws.numel(),
+                                                   c["batch"], 1, logical, c["physical"], torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(y[shift:shift + want_y.numel()].view_as(want_y), want_y)
+    assert not bool(y[:shift].any()) and not bool(y[shift + want_y.numel():].any())
+    assert device_us(dict(c, qkv=moved)) < 4 * device_us(c)
 
 
 def test_rope_access_widths_agree():
