@@ -163,6 +163,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
     const int tile_tokens = kPfRows / group;   // the launch makes sure of group <= 128
     // the tiles with the most keys first, so that the short ones fill the gaps at the end
     const int t0 = int(gridDim.y - 1 - blockIdx.y) * tile_tokens * qtiles, t1 = min(p.tokens, t0 + tile_tokens * qtiles);
+    const int tiles = t0 + tile_tokens < t1 ? qtiles : 1;   // the last block of a sequence may have rows for one tile only
     const int limit = p.logical_pages * p.page_size;
 
     if (threadIdx.x == 0) {
@@ -325,12 +326,14 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
                 good = mbar_wait_suspended(&kv_full[j], 0);
                 tc_fence_after();
 #pragma unroll
-                for (int q = 0; q < qtiles; ++q) scores(j, q);
+                for (int q = 0; q < qtiles; ++q)
+                    if (q < tiles) scores(j, q);
             }
             for (int j = 0; j < steps && good; ++j) {
                 const uint32_t v = v_lo + (j % kPfStages) * kStage;
 #pragma unroll
                 for (int q = 0; q < qtiles; ++q) {
+                    if (q >= tiles) break;
                     good = good && mbar_wait_suspended(&p_full[q * 2 + (j & 1)], (j >> 1) & 1);
                     if (good && q == 0 && j + 2 < steps) good = mbar_wait_suspended(&kv_full[(j + 2) % kPfStages], ((j + 2) / kPfStages) & 1);
                     if (!good) break;
@@ -353,7 +356,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
             mbar_wait_suspended(drained, 0);
         }
         __syncwarp();
-    } else if ((warp >> 2) < qtiles) {
+    } else if ((warp >> 2) < tiles) {
         // -------------------------------------------------------------- softmax
         const int q = warp >> 2, r = (warp & 3) * 32 + lane;
         const uint32_t tm = tmem_base + q * kPfCols + (uint32_t((warp & 3) * 32) << 16);
@@ -505,14 +508,11 @@ bool oss_prefill_takes(const OssAttn& p)
 int oss_prefill_launch(const OssAttn& p, cudaStream_t stream)
 {
     const int tile_tokens = kPfRows / (p.q_heads / p.kv_heads);
-    auto blocks = [&](int qtiles) { return (p.tokens + tile_tokens * qtiles - 1) / (tile_tokens * qtiles); };
-    // Two tiles per CTA keep the exponential unit busy while the other tile's MMAs run; with fewer CTAs than SMs one tile each
-    // uses twice the SMs.
-    const int qtiles = (long long)p.batch * p.kv_heads * blocks(2) >= kSmCount ? 2 : 1;
+    const int qtiles = oss_prefill_tiles(p.batch, p.kv_heads, p.tokens, tile_tokens);
     const auto kernel = qtiles == 2 ? oss_attention_prefill_kernel<2> : oss_attention_prefill_kernel<1>;
     GB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PfSmem::total));
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(unsigned(p.kv_heads), unsigned(blocks(qtiles)), unsigned(p.batch));
+    cfg.gridDim = dim3(unsigned(p.kv_heads), unsigned((p.tokens + tile_tokens * qtiles - 1) / (tile_tokens * qtiles)), unsigned(p.batch));
     cfg.blockDim = dim3(kPfThreads);
     cfg.dynamicSmemBytes = PfSmem::total;
     cfg.stream = stream;

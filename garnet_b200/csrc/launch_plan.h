@@ -50,4 +50,13 @@ inline TcPlan tc_plan(int strips_padded, int chunks, int m)
     return t;
 }
 
+// Query tiles of 128 rows that a CTA of the gpt-oss prefill kernel takes (gpt_oss_prefill.cu); a tile is `tile_tokens` tokens of a
+// kv head's group.  Two keep the exponential unit busy while the other tile's MMAs run, where there is a second tile at all; with
+// fewer CTAs than SMs one tile each uses twice the SMs.
+inline int oss_prefill_tiles(int batch, int kv_heads, int tokens, int tile_tokens)
+{
+    const long long pairs = (tokens + 2 * tile_tokens - 1) / (2 * tile_tokens);
+    return tokens > tile_tokens && batch * (long long)kv_heads * pairs >= kSmCount ? 2 : 1;
+}
+
 }  // namespace gb200

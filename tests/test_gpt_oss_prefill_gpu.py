@@ -192,3 +192,9 @@ def test_queries_that_are_not_bf16_values_stay_on_the_tensor_cores():
     check(c)
     plain, pieces = make(512, [0], 0, seed=10), make(512, [0], 0, exact=False, seed=10)
     assert device_us(pieces) < 4 * device_us(plain)
+
+
+def test_blocks_whose_second_tile_has_no_rows():
+    """Sequences of 33 tokens (two blocks of two tiles, the last with one token) and of 16 (one tile), enough to fill the GPU."""
+    check(make(33, list(range(0, 200, 10)), 0, seed=11))
+    check(make(16, list(range(0, 200, 10)), 0, seed=12))

@@ -15,6 +15,7 @@ extern "C" void tile_plan(int panels, int chunks, int m, int* out)
     out[0] = t.row_tiles, out[1] = t.tile_rows, out[2] = t.kslices;
     for (int s = 0; s <= t.kslices; ++s) out[3 + s] = tc_first_chunk(chunks, t.kslices, s);
 }
+extern "C" int prefill_tiles(int batch, int kv_heads, int tokens, int tile_tokens) { return oss_prefill_tiles(batch, kv_heads, tokens, tile_tokens); }
 """
 SMS = 148
 
@@ -45,3 +46,14 @@ def test_tile_kernel_keeps_its_k_slices_whatever_the_chunk_count(plans, m):
             first = out[3:4 + slices]
             sizes = [b - a for a, b in zip(first, first[1:])]
             assert first[0] == 0 and first[-1] == chunks and min(sizes) >= 1 and max(sizes) - min(sizes) <= 1
+
+
+def test_prefill_takes_a_second_query_tile_only_where_there_is_one(plans):
+    """A CTA takes two tiles when they hold rows and the CTAs still fill the GPU."""
+    plans.prefill_tiles.restype = ctypes.c_int
+    for batch in (1, 2, 3, 7, 20, 64):
+        for kv_heads, tile_tokens in ((8, 16), (1, 16), (8, 128), (2, 42), (16, 1)):
+            for tokens in list(range(1, 70)) + [128, 129, 700, 2048, 65000]:
+                tiles = plans.prefill_tiles(batch, kv_heads, tokens, tile_tokens)
+                blocks = -(-tokens // (2 * tile_tokens))
+                assert tiles == (2 if tokens > tile_tokens and batch * kv_heads * blocks >= SMS else 1)
