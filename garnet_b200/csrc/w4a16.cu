@@ -181,22 +181,17 @@ W4A16::~W4A16()
     if (fault_host) cudaFreeHost(fault_host);
     if (stage_x) cudaFree(stage_x);
     if (stage_y) cudaFree(stage_y);
-    if (stage_ws) cudaFree(stage_ws);
 }
 
-// What callers of the tile kernel (more than 16 rows) are told to bring; the kernel itself no longer needs it.
+// What garnet_b200_w4a16_workspace reports; no kernel uses it.
 size_t W4A16::workspace_bytes(int m) const { return (m > 16 || m > max_rows_per_launch) ? tc_workspace(geo, m) : 0; }
 
-int W4A16::run(const void* d_x, void* d_y, int m, void* ws, size_t ws_bytes, unsigned flags, cudaStream_t stream)
+int W4A16::run(const void* d_x, void* d_y, int m, unsigned flags, cudaStream_t stream)
 {
     if (m <= 0) return fail(GARNET_B200_INVALID_VALUE, "w4a16_run: m must be positive (got %d)", m);
     if (!d_x || !d_y) return fail(GARNET_B200_INVALID_VALUE, "w4a16_run: null x or y");
     if ((reinterpret_cast<uintptr_t>(d_x) & 15) || (reinterpret_cast<uintptr_t>(d_y) & 1))
         return fail(GARNET_B200_INVALID_VALUE, "w4a16_run: x must be 16-byte aligned");
-    // A workspace smaller than garnet_b200_w4a16_workspace asks for (or none) is allowed: the K slices of the tile kernel
-    // meet in distributed shared memory and nothing is written to it.
-    (void)ws;
-    (void)ws_bytes;
     const __nv_bfloat16* x = static_cast<const __nv_bfloat16*>(d_x);
     __nv_bfloat16* y = static_cast<__nv_bfloat16*>(d_y);
     // Above 16 rows the weights are worth expanding once per 128 rows for the tensor core.
@@ -277,8 +272,6 @@ struct HostBatch {
     std::vector<X> xs;
     uint8_t* x_stage = nullptr;
     uint8_t* y_stage = nullptr;
-    void* ws = nullptr;
-    size_t ws_bytes = 0;
     ScatterEntry* table = nullptr;
     int table_count = 0;
     garnet_b200_w4a16_list_t list = nullptr;   // the calls as one persistent launch, when they all share one small batch
@@ -287,7 +280,6 @@ struct HostBatch {
         if (list) garnet_b200_w4a16_list_destroy(list);
         if (x_stage) cudaFree(x_stage);
         if (y_stage) cudaFree(y_stage);
-        if (ws) cudaFree(ws);
         if (table) cudaFree(table);
     }
 };
@@ -475,7 +467,9 @@ int garnet_b200_w4a16_run(garnet_b200_w4a16_t hh, const void* d_x, void* d_y, in
 {
     W4A16* h = reinterpret_cast<W4A16*>(hh);
     if (!h) return fail(GARNET_B200_INVALID_VALUE, "w4a16_run: null handle");
-    return h->run(d_x, d_y, m, d_workspace, workspace_bytes, flags, static_cast<cudaStream_t>(stream));
+    (void)d_workspace;       // any or none: the K slices of the tile kernel meet on the chip
+    (void)workspace_bytes;
+    return h->run(d_x, d_y, m, flags, static_cast<cudaStream_t>(stream));
 }
 
 int garnet_b200_w4a16_run_group(const garnet_b200_w4a16_t* handles, int count, const void* d_x, void* const* d_ys,
@@ -502,7 +496,7 @@ int garnet_b200_w4a16_run_group(const garnet_b200_w4a16_t* handles, int count, c
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (m > max_rows) {   // larger batches: one launch per linear (tile kernel or row blocks)
         for (int g = 0; g < count; ++g)
-            if (int rc = hs[g]->run(d_x, ys[g], m, nullptr, 0, flags, s)) return rc;
+            if (int rc = hs[g]->run(d_x, ys[g], m, flags, s)) return rc;
         return GARNET_B200_OK;
     }
     return W4A16::launch_stream_group(hs, count, static_cast<const __nv_bfloat16*>(d_x), ys, ldys, m, flags, s);
@@ -519,20 +513,17 @@ static void* device_alias_of(const void* host_ptr)
     return attr.type == cudaMemoryTypeHost ? attr.devicePointer : nullptr;
 }
 
-// Device staging for the host-buffer calls of one handle (x, y and workspace for up to
-// `m` rows).  Allocates; the run calls do not.
+// Device staging for the host-buffer calls of one handle (x and y for up to `m` rows).  Allocates; the run calls do not.
 static int reserve_host(W4A16* h, int m)
 {
     if (m <= h->stage_rows) return GARNET_B200_OK;
     if (h->stage_x) cudaFree(h->stage_x);
     if (h->stage_y) cudaFree(h->stage_y);
-    if (h->stage_ws) cudaFree(h->stage_ws);
-    h->stage_x = h->stage_y = h->stage_ws = nullptr;
+    h->stage_x = h->stage_y = nullptr;
     h->stage_rows = 0;
-    const size_t xb = size_t(m) * h->geo.cols * 2, yb = size_t(m) * h->geo.rows * 2, wb = h->workspace_bytes(m);
+    const size_t xb = size_t(m) * h->geo.cols * 2, yb = size_t(m) * h->geo.rows * 2;
     GB_CUDA(cudaMalloc(&h->stage_x, xb));
     GB_CUDA(cudaMalloc(&h->stage_y, yb));
-    if (wb) GB_CUDA(cudaMalloc(&h->stage_ws, wb));
     h->stage_rows = m;
     return GARNET_B200_OK;
 }
@@ -544,7 +535,7 @@ static int run_host_one(W4A16* h, const void* h_x, void* h_y, int m, cudaStream_
         return fail(GARNET_B200_INVALID_VALUE,
                     "w4a16_run_host: %d rows but staging is reserved for %d: call garnet_b200_w4a16_reserve_host first", m,
                     h->stage_rows);
-    const size_t xb = size_t(m) * h->geo.cols * 2, yb = size_t(m) * h->geo.rows * 2, wb = h->workspace_bytes(m);
+    const size_t xb = size_t(m) * h->geo.cols * 2, yb = size_t(m) * h->geo.rows * 2;
     // y in pinned, mapped host memory is written by the kernel itself (one posted write per
     // output over the host link, no copy to enqueue); any other y goes through a staged copy.
     // The lookup is a host-side query and is repeated on every call: the same address may be
@@ -552,7 +543,7 @@ static int run_host_one(W4A16* h, const void* h_x, void* h_y, int m, cudaStream_
     void* alias = device_alias_of(h_y);
     GB_CUDA(cudaMemcpyAsync(h->stage_x, h_x, xb, cudaMemcpyHostToDevice, s));
     void* y_dev = alias ? alias : h->stage_y;
-    if (int rc = h->run(h->stage_x, y_dev, m, h->stage_ws, wb, 0, s)) return rc;
+    if (int rc = h->run(h->stage_x, y_dev, m, 0, s)) return rc;
     if (!alias) GB_CUDA(cudaMemcpyAsync(h_y, h->stage_y, yb, cudaMemcpyDeviceToHost, s));
     return GARNET_B200_OK;
 }
@@ -577,12 +568,11 @@ int garnet_b200_w4a16_batch_create(const garnet_b200_w4a16_t* handles, const voi
     if (!handles || !h_xs || !h_ys || !ms || !out || count <= 0)
         return fail(GARNET_B200_INVALID_VALUE, "w4a16_batch_create: bad argument");
     std::unique_ptr<HostBatch> b(new HostBatch);
-    size_t x_total = 0, y_total = 0, ws_max = 0;
+    size_t x_total = 0, y_total = 0;
     for (int i = 0; i < count; ++i) {
         W4A16* h = reinterpret_cast<W4A16*>(handles[i]);
         if (!h || !h_xs[i] || !h_ys[i] || ms[i] <= 0)
             return fail(GARNET_B200_INVALID_VALUE, "w4a16_batch_create: bad argument at index %d", i);
-        ws_max = std::max(ws_max, h->workspace_bytes(ms[i]));
         const size_t xb = size_t(ms[i]) * h->geo.cols * 2, yb = size_t(ms[i]) * h->geo.rows * 2;
         // inputs are read-only during a run: every distinct host buffer is copied once
         int slot = -1;
@@ -598,8 +588,6 @@ int garnet_b200_w4a16_batch_create(const garnet_b200_w4a16_t* handles, const voi
     }
     GB_CUDA(cudaMalloc(&b->x_stage, x_total));
     GB_CUDA(cudaMalloc(&b->y_stage, y_total));
-    if (ws_max) GB_CUDA(cudaMalloc(&b->ws, ws_max));   // the calls run one after the other: one workspace serves them all
-    b->ws_bytes = ws_max;
     // Calls that all have the same small batch run as one list (one launch for the lot).
     bool one_list = true;
     for (const HostBatch::Call& c : b->calls)
@@ -644,7 +632,7 @@ int garnet_b200_w4a16_batch_run(garnet_b200_w4a16_batch_t bb, void* stream)
         if (int rc = garnet_b200_w4a16_list_run(b->list, 0, stream)) return rc;
     } else {
         for (const HostBatch::Call& c : b->calls)
-            if (int rc = c.h->run(b->x_stage + b->xs[c.x_slot].off, b->y_stage + c.y_off, c.m, b->ws, b->ws_bytes, 1, s)) return rc;
+            if (int rc = c.h->run(b->x_stage + b->xs[c.x_slot].off, b->y_stage + c.y_off, c.m, 1, s)) return rc;
     }
     if (b->table_count) {
         cudaLaunchConfig_t cfg = {};

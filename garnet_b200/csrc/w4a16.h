@@ -25,7 +25,6 @@ struct W4A16 {
     // staging for the host-buffer entry point
     void* stage_x = nullptr;
     void* stage_y = nullptr;
-    void* stage_ws = nullptr;
     int stage_rows = 0;
 
     ~W4A16();
@@ -37,7 +36,7 @@ struct W4A16 {
                                    const int* ldys, int m, unsigned flags, cudaStream_t stream);
     int init_tc();
     int launch_tc(const __nv_bfloat16* x, __nv_bfloat16* y, int m, unsigned flags, cudaStream_t stream);
-    int run(const void* d_x, void* d_y, int m, void* ws, size_t ws_bytes, unsigned flags, cudaStream_t stream);
+    int run(const void* d_x, void* d_y, int m, unsigned flags, cudaStream_t stream);
 };
 
 size_t tc_workspace(const PackGeom& geo, int m);

@@ -458,8 +458,8 @@ w4a16_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap x_map, con
 
 // ------------------------------------------------------------------ host side
 
-// Workspace that a call of m rows is told to bring: fp32 partial sums of the K slices, which now meet on the chip.  The size
-// stays what callers were told before.
+// The size that garnet_b200_w4a16_workspace reports: the fp32 partial sums of the plan that once met in global memory.  Nothing
+// uses such a workspace; the reported size is part of the interface.
 size_t tc_workspace(const PackGeom& geo, int m)
 {
     const int row_tiles = (m + 127) / 128, panels256 = (geo.strips_padded + 15) / 16;

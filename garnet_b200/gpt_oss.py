@@ -47,7 +47,7 @@ def attention(opt, qkv, keys, values, table, lengths, starts, active, sinks, bat
     if ws is None:
         need = ctypes.c_size_t(0)
         check(lib().garnet_b200_gpt_oss_attention_workspace(ctypes.byref(opt), batch, logical_pages, ctypes.byref(need)))
-        ws = torch.zeros(need.value, dtype=torch.uint8, device=qkv.device)
+        ws = torch.empty(need.value, dtype=torch.uint8, device=qkv.device)
     ops = _Operands(qkv.data_ptr(), keys.data_ptr(), values.data_ptr(), table.data_ptr(), lengths.data_ptr(), starts.data_ptr(),
                     active.data_ptr(), sinks.data_ptr())
     check(lib().garnet_b200_gpt_oss_attention(ctypes.byref(opt), ops, y.data_ptr(), ws.data_ptr(), ws.numel(), batch, tokens,

@@ -167,8 +167,6 @@ class W4A16Linear:
         self._h = ctypes.c_void_p(None)
         self.n = self.k = self.group = 0
         self._keep = None
-        self._ws = None
-        self._ws_need = (-1, 0)          # (rows, workspace bytes) of the last call
         self._host_rows = 0
 
     def reserve_host(self, max_m: int) -> None:
@@ -210,17 +208,6 @@ class W4A16Linear:
         check(lib().garnet_b200_w4a16_workspace(self._h, m, ctypes.byref(out)))
         return out.value
 
-    def _workspace(self, m: int, device) -> torch.Tensor | None:
-        rows, need = self._ws_need
-        if rows != m:
-            need = self.workspace_bytes(m)
-            self._ws_need = (m, need)
-        if need == 0:
-            return None
-        if self._ws is None or self._ws.numel() < need or self._ws.device != device:
-            self._ws = torch.empty(need, dtype=torch.uint8, device=device)
-        return self._ws
-
     # Q4Q8Linear::Forward (q4q8_linear.cpp:315-389)
     def forward(self, x: torch.Tensor, out: torch.Tensor | None = None, workspace: torch.Tensor | None = None,
                 pdl: bool = True) -> torch.Tensor:
@@ -229,10 +216,9 @@ class W4A16Linear:
         x2 = _rows(x, self.k)
         m = x2.shape[0]
         y = out if out is not None else torch.empty(m, self.n, dtype=torch.bfloat16, device=x.device)
-        ws = workspace if workspace is not None else self._workspace(m, x.device)
         check(lib().garnet_b200_w4a16_run(self._h, x2.data_ptr(), y.data_ptr(), m,
-                                          ws.data_ptr() if ws is not None else None,
-                                          ws.numel() if ws is not None else 0, 1 if pdl else 0, stream_ptr()))
+                                          workspace.data_ptr() if workspace is not None else None,
+                                          workspace.numel() if workspace is not None else 0, 1 if pdl else 0, stream_ptr()))
         return y
 
     def forward_host(self, x_host: torch.Tensor, y_host: torch.Tensor) -> torch.Tensor:
@@ -263,8 +249,6 @@ class W4A16Linear:
             lib().garnet_b200_w4a16_destroy(self._h)
             self._h = ctypes.c_void_p(None)
         self._keep = None
-        self._ws = None
-        self._ws_need = (-1, 0)
         self._host_rows = 0
 
     def __del__(self):

@@ -127,7 +127,8 @@ int garnet_b200_w4a16_create_prepacked(const uint8_t* d_packed, int scale_dtype,
 /* Logical rows held by this handle (N / shard_world) and K. */
 int garnet_b200_w4a16_shape(garnet_b200_w4a16_t h, int* n_local, int* k);
 
-/* Workspace bytes `run` needs for a batch of m rows (0 is possible). */
+/* Workspace bytes that a caller may bring to `run` for a batch of m rows (0 up to 16 rows).  `run` takes a workspace of any
+ * size or none and writes nothing to it: partial sums meet on the chip. */
 int garnet_b200_w4a16_workspace(garnet_b200_w4a16_t h, int m, size_t* bytes);
 
 /* y[m, n_local] = x[m, k] W^T.  x, y bf16 device pointers, row-major, 16-byte
@@ -360,7 +361,8 @@ int garnet_b200_gpt_oss_rope(const garnet_b200_gpt_oss_options* options, const f
  * lengths int32 [batch], starts int32 [batch], active int32 [batch], sinks f32 [q heads]: appends the
  * rows' k and v at positions starts[b] + t, then y[row, head] = softmax over the visible window, with
  * the head's sink in the denominator only (RunGptOssAttention, gpt_oss_kernels.cu:1012-1210).
- * The workspace (zero-filled once by the caller) is needed at decode (tokens == 1, prefill == 0). */
+ * A decode call (tokens == 1, prefill == 0) of 64-wide heads in groups of up to 16 has to bring a workspace of the reported
+ * size on a 256-byte boundary; its contents do not matter and are left alone.  Other calls need none. */
 int garnet_b200_gpt_oss_attention_workspace(const garnet_b200_gpt_oss_options* options, int batch, int logical_pages, size_t* bytes);
 int garnet_b200_gpt_oss_attention(const garnet_b200_gpt_oss_options* options, const void* const* in, float* d_y, void* d_workspace,
                                   size_t workspace_bytes, int batch, int tokens, int logical_pages, int physical_pages, void* stream);
