@@ -285,8 +285,9 @@ bool oss_decode_takes(const OssAttn& p)
 
 int oss_decode_launch(const OssAttn& p, cudaStream_t stream)
 {
-    // As many CTAs per (sequence, kv head) as have a tile for each of their warps; above four CTAs per SM the clusters shrink.
-    // With more CTAs than SMs a CTA has four warps, so that three fit an SM (64 KiB of rings); else eight.
+    // As many CTAs per (sequence, kv head) as have a tile for each of their warps; a grid of more than eight CTAs per SM, which is
+    // well over two waves, gets smaller clusters.  With more CTAs than SMs a CTA has four warps, so that three fit an SM (64 KiB of
+    // rings, 168 registers); else eight.
     const long long span = (long long)p.logical_pages * p.page_size, seen = p.window ? std::min<long long>(p.window, span) : span;
     const long long pairs = (long long)p.batch * p.kv_heads;
     int splits = kDecMaxSplits;

@@ -64,33 +64,6 @@ __device__ __forceinline__ float ex2(float x)
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// MMAs whose descriptors arrive as their low words (start address; the high word is the constant of umma_desc_k_sw128): an
-// addition of a constant per MMA.  The issuing thread shares its scheduler with softmax warps, and rebuilding 64-bit
-// descriptors cost it about 100 clocks per MMA, two to three times what the tensor pipe needs for one.
-constexpr uint32_t kPfDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
-__device__ __forceinline__ uint32_t desc_lo(uint32_t smem_addr) { return ((smem_addr & 0x3FFFFu) >> 4) | (1u << 16); }
-// D[tmem] (+)= A[smem] * B[smem]
-__device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, bool accumulate)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
-        "mov.b64 a, {%1, %5};\n\tmov.b64 b, {%2, %5};\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t}" ::"r"(d_tmem),
-        "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(uint32_t(accumulate)), "n"(kPfDescHi)
-        : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem]
-__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc, bool accumulate)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\t"
-        "mov.b64 b, {%2, %5};\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n\t}" ::"r"(d_tmem),
-        "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(uint32_t(accumulate)), "n"(kPfDescHi)
-        : "memory");
-}
 __device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const uint32_t (&r)[8])
 {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
@@ -307,7 +280,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
         if (elect_one()) {
             constexpr uint32_t idesc_qk = umma_idesc_f16(1, kPfRows, kPfKeys);
             constexpr uint32_t idesc_pv = umma_idesc_f16(1, kPfRows, kOssDim) | (1u << 16);   // V: MN-major
-            const uint32_t q_lo = desc_lo(smem_u32(q_tiles)), k_lo = desc_lo(smem_u32(kv_ring)), v_lo = desc_lo(smem_u32(kv_ring + kPfKvBytes));
+            const uint32_t q_lo = umma_desc_lo(smem_u32(q_tiles)), k_lo = umma_desc_lo(smem_u32(kv_ring)), v_lo = umma_desc_lo(smem_u32(kv_ring + kPfKvBytes));
             constexpr uint32_t kStage = 2 * kPfKvBytes >> 4;
             // scores of step j of tile q, into set j & 1
             const auto scores = [&](int j, int q) {
@@ -317,7 +290,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
                 for (int piece = q_pieces - 1; piece >= 0; --piece) {
 #pragma unroll
                     for (int k16 = 0; k16 < kOssDim / 16; ++k16)
-                        umma_ss(d, a + piece * (2 * kPfTileBytes >> 4) + k16 * 2, k + k16 * 2, idesc_qk, piece + 1 < q_pieces || k16 > 0);
+                        umma_f16_ss(d, a + piece * (2 * kPfTileBytes >> 4) + k16 * 2, k + k16 * 2, idesc_qk, piece + 1 < q_pieces || k16 > 0);
                 }
                 umma_commit(&s_full[q * 2 + (j & 1)]);
             };
@@ -344,7 +317,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) oss_attention_prefill_kernel(co
                     for (int piece = 0; piece < 3; ++piece)
 #pragma unroll
                         for (int k16 = 0; k16 < kPfKeys / 16; ++k16)
-                            umma_ts(tile + kPfColPv, pieces[piece] + k16 * 8, v + k16 * (2048 >> 4), idesc_pv, piece > 0 || k16 > 0);
+                            umma_f16_ts(tile + kPfColPv, pieces[piece] + k16 * 8, v + k16 * (2048 >> 4), idesc_pv, piece > 0 || k16 > 0);
                     umma_commit(&pv_full[q]);
                     if (j + 2 < steps) scores(j + 2, q);
                 }

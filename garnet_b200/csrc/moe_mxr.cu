@@ -263,11 +263,11 @@ moe_mxr_kernel(const RxParams p, const __grid_constant__ CUtensorMap w_map, cons
         if (elect_one()) {
             uint32_t s = 0, phase = 0, it_n = 0;
             bool good = true;
-            // The issuing thread shares its scheduler with two epilogue warps, so its loop is kept to a few instructions per
+            // The issuing thread shares its scheduler with four epilogue warps, so its loop is kept to a few instructions per
             // MMA: stage-0 descriptors plus a stage offset plus constants, and four instruction descriptors that differ only
             // in the scale selectors.
             const uint32_t ring_addr = smem_u32(ring);
-            const uint32_t hi_d0 = mx_desc_lo(ring_addr), lo_d0 = mx_desc_lo(ring_addr + kRxATile), w_d0 = mx_desc_lo(ring_addr + 2 * kRxATile);
+            const uint32_t hi_d0 = umma_desc_lo(ring_addr), lo_d0 = umma_desc_lo(ring_addr + kRxATile), w_d0 = umma_desc_lo(ring_addr + 2 * kRxATile);
             const uint32_t sfx_d0 = mx_plain_lo(ring_addr + 2 * kRxATile + kRxBTile);
             constexpr uint32_t kStageUnits = kRxStageBytes >> 4, kAtomUnits = kMxAtom >> 4;
             // A = e4m3 pieces (rows), B = e2m1 weights

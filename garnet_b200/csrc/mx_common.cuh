@@ -14,11 +14,6 @@ __host__ __device__ constexpr int mx_tile_box(int rows) { return rows <= kMxBoxS
 
 #if defined(__CUDACC__)
 
-// Descriptors travel as their low words (start address in 16-byte units); the high words are constants, so that the thread
-// that issues the MMAs - it shares its scheduler with epilogue warps - adds one constant per operand and MMA.
-// K-major operand, 128-byte swizzle (umma_desc_k_sw128):
-constexpr uint32_t kMxDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
-__device__ __forceinline__ uint32_t mx_desc_lo(uint32_t smem_addr) { return ((smem_addr & 0x3FFFFu) >> 4) | (1u << 16); }
 // K-major operand without swizzle: 8-row core matrices of 128 contiguous bytes, 128 bytes apart (the source format of the
 // scale-atom copies):
 constexpr uint32_t kMxPlainHi = (128u >> 4) | (1u << 14);
@@ -52,20 +47,10 @@ __device__ __forceinline__ void umma_mx(uint32_t d_tmem, uint32_t a_lo, uint32_t
         "mov.b64 a, {%1, %7};\n\tmov.b64 b, {%2, %7};\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], a, b, %3, [%5], [%6], p;\n\t}" ::"r"(d_tmem),
-        "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(uint32_t(accumulate)), "r"(sfa), "r"(sfb), "n"(kMxDescHi)
+        "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(uint32_t(accumulate)), "r"(sfa), "r"(sfb), "n"(kDescHiSw128)
         : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
-{
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr)
-        : "memory");
-}
 __device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t (&r)[8])
 {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"

@@ -25,8 +25,6 @@ int make_tensor_map_2d_bytes(CUtensorMap* map, const void* base, uint64_t rows, 
 
 #if defined(__CUDACC__)
 
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity) { return mbar_wait(bar, parity); }
-
 __device__ __forceinline__ bool elect_one()
 {
     uint32_t pred;
@@ -74,18 +72,12 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols)
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, rows of 128
-// bytes, 8-row groups 1024 bytes apart; descriptor version 1 (Blackwell).
-__device__ __forceinline__ uint64_t umma_desc_k_sw128(uint32_t smem_addr)
-{
-    uint64_t d = 0;
-    d |= uint64_t((smem_addr & 0x3FFFFu) >> 4);   // start address
-    d |= uint64_t(1) << 16;                       // leading byte offset (unused for swizzled K-major)
-    d |= uint64_t(1024 >> 4) << 32;               // stride byte offset: 8 rows * 128 B
-    d |= uint64_t(1) << 46;                       // version
-    d |= uint64_t(2) << 61;                       // SWIZZLE_128B
-    return d;
-}
+// Shared-memory matrix descriptors travel as their low words; the high words are constants, so that the thread that issues the
+// MMAs, which shares its scheduler with busy warps, adds one constant per operand and MMA (rebuilding 64-bit descriptors cost it
+// about 100 clocks per MMA, two to three times what the tensor pipe needs for one).
+// 128-byte swizzle, rows of 128 bytes, 8-row groups 1024 bytes apart; descriptor version 1 (Blackwell):
+constexpr uint32_t kDescHiSw128 = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t umma_desc_lo(uint32_t smem_addr) { return ((smem_addr & 0x3FFFFu) >> 4) | (1u << 16); }
 
 // Instruction descriptor for kind::f16: fp32 accumulate, A and B K-major.
 // fmt: 0 = fp16, 1 = bf16.
@@ -94,14 +86,25 @@ __host__ __device__ constexpr uint32_t umma_idesc_f16(int fmt, int m, int n)
     return (1u << 4) | (uint32_t(fmt) << 7) | (uint32_t(fmt) << 10) | (uint32_t(n >> 3) << 17) | (uint32_t(m >> 4) << 24);
 }
 
-// D[tmem] (+)= A[smem] * B[smem]; issued by one thread.
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, bool accumulate)
+// D[tmem] (+)= A * B, issued by one thread: both from shared memory, or A from tensor memory.
+__device__ __forceinline__ void umma_f16_ss(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, bool accumulate)
 {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+        "mov.b64 a, {%1, %5};\n\tmov.b64 b, {%2, %5};\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(uint32_t(accumulate))
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t}" ::"r"(d_tmem),
+        "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(uint32_t(accumulate)), "n"(kDescHiSw128)
+        : "memory");
+}
+__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc, bool accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\t"
+        "mov.b64 b, {%2, %5};\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n\t}" ::"r"(d_tmem),
+        "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(uint32_t(accumulate)), "n"(kDescHiSw128)
         : "memory");
 }
 
@@ -132,6 +135,16 @@ __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32])
           "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
           "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
           "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr)
         : "memory");
 }

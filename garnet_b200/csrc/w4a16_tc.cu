@@ -48,7 +48,6 @@ constexpr int kTcHalfRows = 128;
 static_assert(2 * kTcMaxRows + kTcAStages * kTcACols <= 512 && kTcHalfRows + kTcAStages * kTcACols <= 256, "tensor memory");
 
 struct TcParams {
-    const uint8_t* packed;
     __nv_bfloat16* y;
     int* fault;
     int m, n;
@@ -115,20 +114,6 @@ __device__ __forceinline__ uint4 int4_word_to_bf16x8_f32(uint32_t w, float s)
     return make_uint4(out[0], out[1], out[2], out[3]);
 }
 
-// D[tmem] (+)= A[tmem] * B[smem]; the descriptor comes as its low word (tc_desc_lo), so that the issuing thread adds one
-// constant per MMA.
-constexpr uint32_t kTcDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
-__device__ __forceinline__ uint32_t tc_desc_lo(uint32_t smem_addr) { return ((smem_addr & 0x3FFFFu) >> 4) | (1u << 16); }
-__device__ __forceinline__ void tc_umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc, bool accumulate)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\t"
-        "mov.b64 b, {%2, %5};\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n\t}" ::"r"(d_tmem),
-        "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(uint32_t(accumulate)), "n"(kTcDescHi)
-        : "memory");
-}
 __device__ __forceinline__ void tc_st_32x32(uint32_t taddr, const uint4 (&v)[8])
 {
     asm volatile(
@@ -140,17 +125,6 @@ __device__ __forceinline__ void tc_st_32x32(uint32_t taddr, const uint4 (&v)[8])
         "r"(v[7].z), "r"(v[7].w)
         : "memory");
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tc_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
-{
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr)
-        : "memory");
-    tmem_ld_wait();
 }
 // y[row, n], y[row, n + 1] of a pair of neighbouring outputs.
 __device__ __forceinline__ void tc_store_pair(const TcParams& p, int row, int n, float a, float b, bool wide)
@@ -290,7 +264,7 @@ w4a16_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap x_map, con
             bool good = true;
             // UMMA M = 128 weight rows (TMEM lanes), N = the tile's batch rows (TMEM columns)
             const uint32_t idesc = umma_idesc_f16(1, 128, p.tile_rows);
-            const uint32_t b0 = tc_desc_lo(smem_u32(b_ring));
+            const uint32_t b0 = umma_desc_lo(smem_u32(b_ring));
             for (int item = blockIdx.x; item < items && good; item += gridDim.x, ++it_n) {
                 const uint32_t buf = it_n & 1;
                 if (it_n >= 2 && !mbar_wait_suspended(&acc_empty[buf], ((it_n >> 1) - 1) & 1)) {
@@ -311,7 +285,7 @@ w4a16_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap x_map, con
                     tc_fence_after();
                     const uint32_t a = tmem_base + p.col_a + s * kTcACols, b = b0 + sb * (p.tile_rows * 128 >> 4);
 #pragma unroll
-                    for (int k16 = 0; k16 < 4; ++k16) tc_umma_ts(d, a + k16 * 8, b + k16 * 2, idesc, kt > 0 || k16 > 0);
+                    for (int k16 = 0; k16 < 4; ++k16) umma_f16_ts(d, a + k16 * 8, b + k16 * 2, idesc, kt > 0 || k16 > 0);
                     umma_commit(&a_empty[s]);    // stages reusable once these MMAs have read them
                     umma_commit(&b_empty[sb]);
                     if (++s == kTcAStages) s = 0, a_phase ^= 1;
@@ -399,7 +373,8 @@ w4a16_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap x_map, con
             const uint32_t taddr = tmem_base + (uint32_t(quarter * 32) << 16) + buf * kTcMaxRows;
             for (int c0 = 0; c0 < rows; c0 += 16) {
                 uint32_t v[16];
-                tc_ld_32x16(taddr + c0, v);
+                tmem_ld_32x16(taddr + c0, v);
+                tmem_ld_wait();
                 if (p.kslices > 1) {
                     float* part = reinterpret_cast<float*>(b_ring) + size_t(c0) * 128 + quarter * 32 + lane;
 #pragma unroll
@@ -533,7 +508,6 @@ int W4A16::launch_tc(const __nv_bfloat16* x, __nv_bfloat16* y, int m, unsigned f
     CUtensorMap map;
     if (int rc = make_tensor_map_2d_16bit(&map, x, uint64_t(m), uint64_t(geo.cols), uint32_t(plan.tile_rows))) return rc;
     TcParams p;
-    p.packed = packed;
     p.y = y;
     p.fault = fault_dev;
     p.m = m;
