@@ -13,8 +13,8 @@
 //   2 x 4 softmax     one thread per query row: 64 scores into registers, running maximum (the sink is its first value),
 //   warps             p = 2^(s c - m c), the row's sum in fp32, P over the scores in tensor memory; the P V of the step before
 //                     is added to O, which stays in registers and is rescaled only when a row's maximum has grown by more than
-//                     2^8 since the last time (the final division makes that exact).  The fp32 work runs two values per
-//                     instruction (f32x2).
+//                     2^8 since the last time (the final division makes that exact; the conditional rescaling of
+//                     FlashAttention-4).  The fp32 work runs two values per instruction (f32x2).
 // Numerics: the queries are bf16-valued fp32, so Q K^T has exact products; the queries of a CTA that holds others enter as three
 // bf16 numbers each.  P is fp32 and enters the MMA as three bf16 numbers, which hold eight of its 24 bits each.  The tensor core
 // truncates what it accumulates, so a sum that stays in it loses about half a unit of its last place per MMA: each step starts a
@@ -24,9 +24,10 @@
 // meet a zero piece) is computed again by the row loop.
 //
 // Bound: per 128 x 64 scores the tensor pipe needs about 600 clocks (12 P V MMAs at 33, 4 Q K^T MMAs at 50) and the exponentials
-// 512 (16 per clock and SM); most of a step's time goes into the instruction issue of the schedulers that a loader or the MMA warp
-// shares with two softmax warps.
-// 2048 tokens, 64 / 8 heads (events, append included): 132 us; 110 us with two pieces of P and O in tensor memory, whose sums
+// 512 (16 per clock and SM).  Neither is what it waits for: at 2048 tokens the tensor pipe is 23 % busy and the issue slots 44 %
+// (ncu), and a warp spends its time on fixed latencies and on tensor memory and barriers: the chain of a tile's step (scores ->
+// maximum -> exponentials -> pieces -> P V) with one other tile on the SM to hide it.
+// 2048 tokens, 64 / 8 heads (events, append included): 131 us; 110 us with two pieces of P and O in tensor memory, whose sums
 // were worse than the row loop's; pieces rounded instead of cut off 135 us, stored 32 keys at a time 141 us.
 #include <algorithm>
 #include <cfloat>

@@ -16,10 +16,10 @@
 // Bound: an MMA of N columns takes N / 2 clocks and reads N x 32 bytes; expanding through shared memory instead (the form
 // before: 32 KiB written and 48 KiB read per 128 x 256 x 64 step, a proxy fence per warp and step) took 1535 clocks per step
 // against 512 of MMAs.  Batch tiles are even shares of the batch in multiples of 16 rows, so little of them is padding.
-//   rows x K -> N             before      now (called from Python; x [1000, 2048]: 825 TFLOP/s)
-//   1000 x 2048 -> 12288      75.0 us     61.0 us
-//     77 x 2048 -> 4096       15.6 us     9.7 us
-//     16 x 6144 -> 2048       17.6 us     8.3 us
+//   rows x K -> N             before      now (called from Python; x [1000, 2048]: 829 TFLOP/s)
+//   1000 x 2048 -> 12288      74.3 us     60.7 us
+//     77 x 2048 -> 4096       15.6 us     9.5 us
+//     16 x 6144 -> 2048       17.6 us     8.0 us
 // Numerics: w = bf16(q * s) (one rounding of the dequantised weight), products
 // exact, fp32 accumulation in TMEM, bf16 output.
 #include <algorithm>
